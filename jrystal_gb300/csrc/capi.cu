@@ -7,14 +7,15 @@
 #include <cstring>
 #include <string>
 #include <vector>
+#include "fast_dispatch.h"
 #include "plan.h"
 
 namespace jrg {
 
 // ---- launchers implemented in the kernel files ----
-template <typename R> int launch_plane_inv_sphere(const jrg_plan*, const void*, void*, int, cudaStream_t);
+template <typename R> int launch_plane_inv_sphere(const jrg_plan*, const void*, void*, int, const double*, cudaStream_t);
 template <typename R> int launch_line_density(const jrg_plan*, const void*, void*, const double*, double, int, int, int, double*, cudaStream_t);
-template <typename R> int launch_line_apply_v(const jrg_plan*, const void*, void*, const void*, int, int, cudaStream_t);
+template <typename R> int launch_line_apply_v(const jrg_plan*, const void*, void*, const void*, int, int, const double*, cudaStream_t);
 template <typename R> int launch_plane_fwd_sphere(const jrg_plan*, const void*, const void*, void*, const double*, int, int, double, cudaStream_t);
 template <typename R> int launch_fft3d_dense(const FftAxis*, const C_t<R>*, int, int, bool, const void*, C_t<R>*, C_t<R>*, double, cudaStream_t);
 template <typename R> int launch_pack_params(const void*, const void*, void*, int, int, int, bool, cudaStream_t);
@@ -242,7 +243,7 @@ int jrg_plan_destroy(jrg_plan* P) {
   if (!P) return JRG_OK;
   void* ptrs[] = {P->d.gidx, P->d.sph_yz, P->d.plane_x, P->d.plane_off, P->d.row_off, P->d.rows,
                   P->d.xact, P->d.tk, P->d.tkf, P->d.tw, P->d.vext, P->d.ginv, P->d.gvec, P->d.proj,
-                  P->d.rowmap};
+                  P->d.rowmap, P->d.xmap, P->d.col_of};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (P->prec == 32 && P->d.vext64) cudaFree(P->d.vext64);
@@ -336,18 +337,6 @@ int jrg_plan_create(const jrg_plan_desc* d, jrg_plan** out) {
   }
   plane_off.push_back(ng);
   row_off.push_back((int)rows.size());
-  // dense map of every active row: sphere index per z, -1 off the sphere
-  std::vector<int> rowmap(rows.size() * (size_t)P->nz, -1);
-  {
-    size_t r = 0;
-    for (int e = 0; e < ng; ++e) {
-      const int x = (int)(gidx[e] / nyz), y = sph_yz[e] / P->nz, z = sph_yz[e] % P->nz;
-      const int pl = xact[x];
-      if (r < (size_t)row_off[pl]) r = row_off[pl];
-      while (rows[r] != y) ++r;    // rows of a plane are increasing, as the sphere order is
-      rowmap[r * P->nz + z] = e;
-    }
-  }
   P->nact = (int)plane_x.size();
   {
     auto mid = [](int i, int n) { return i >= n / 4 && i < 3 * n / 4; };   // the zero blocks
@@ -359,6 +348,56 @@ int jrg_plan_create(const jrg_plan_desc* d, jrg_plan** out) {
     for (int e = 0; e < ng; ++e) {
       const int y = sph_yz[e] / P->nz, z = sph_yz[e] % P->nz;
       if (mid(y, P->ny) || mid(z, P->nz)) P->yzprune = false;
+    }
+  }
+  // column-first transforms: the (y, z) columns of the sphere in (y, z) order,
+  // their sphere entries per x, both indexed by window position (|i| < N/4
+  // when the whole sphere lies there, else every index)
+  std::vector<int> xmap;
+  std::vector<short> col_of;
+  {
+    auto out = [](int i, int n) { const int h = (n - 1) / 4; return i > h && i < n - h; };
+    P->colwin = true;
+    std::vector<int> id((size_t)nyz, -1);
+    for (int e = 0; e < ng; ++e) {
+      const int x = (int)(gidx[e] / nyz), y = sph_yz[e] / P->nz, z = sph_yz[e] % P->nz;
+      if (out(x, P->nx) || out(y, P->ny) || out(z, P->nz)) P->colwin = false;
+      id[sph_yz[e]] = 0;
+    }
+    P->ncol = 0;
+    for (int& c : id)
+      if (c == 0) c = P->ncol++;
+    const int per16 = 16 / csize(P->prec);
+    P->tpitch = (P->ncol + per16 - 1) / per16 * per16;
+    P->cols = P->ncol < 32768 && (long long)P->nx * P->tpitch <= (long long)P->nact * nyz &&
+              cols::covers(P->prec, P->nx, P->ny, P->nz, P->nb, P->colwin,
+                            P->xprune && P->yzprune && P->nx == P->ny);
+    if (P->cols) {
+      auto size = [&](int n) { return P->colwin ? 2 * ((n - 1) / 4) + 1 : n; };
+      auto pos = [&](int i, int n) { return (!P->colwin || i <= (n - 1) / 4) ? i : i - (n - size(n)); };
+      const int wz = size(P->nz);
+      xmap.assign((size_t)size(P->nx) * P->ncol, -1);
+      col_of.assign((size_t)size(P->ny) * wz, -1);
+      for (int e = 0; e < ng; ++e) {
+        const int x = (int)(gidx[e] / nyz), y = sph_yz[e] / P->nz, z = sph_yz[e] % P->nz;
+        const int c = id[sph_yz[e]];
+        xmap[(size_t)pos(x, P->nx) * P->ncol + c] = e;
+        col_of[(size_t)pos(y, P->ny) * wz + pos(z, P->nz)] = (short)c;
+      }
+    }
+  }
+  // dense map of every active row: sphere index per z, -1 off the sphere (the
+  // plane-first kernels' gather)
+  std::vector<int> rowmap;
+  if (!P->cols) {
+    rowmap.assign(rows.size() * (size_t)P->nz, -1);
+    size_t r = 0;
+    for (int e = 0; e < ng; ++e) {
+      const int x = (int)(gidx[e] / nyz), y = sph_yz[e] / P->nz, z = sph_yz[e] % P->nz;
+      const int pl = xact[x];
+      if (r < (size_t)row_off[pl]) r = row_off[pl];
+      while (rows[r] != y) ++r;    // rows of a plane are increasing, as the sphere order is
+      rowmap[r * P->nz + z] = e;
     }
   }
   P->max_rows = 0;
@@ -412,7 +451,12 @@ int jrg_plan_create(const jrg_plan_desc* d, jrg_plan** out) {
 #define UP(field, vec) \
   if (!rc) rc = up((void**)&P->d.field, vec.data(), vec.size() * sizeof(vec[0]));
   UP(gidx, gidx) UP(sph_yz, sph_yz) UP(plane_x, plane_x) UP(plane_off, plane_off)
-  UP(row_off, row_off) UP(rows, rows) UP(xact, xact) UP(tk, tk) UP(tkf, tkf) UP(rowmap, rowmap)
+  UP(row_off, row_off) UP(rows, rows) UP(xact, xact) UP(tk, tk) UP(tkf, tkf)
+  if (P->cols) {
+    UP(xmap, xmap) UP(col_of, col_of)
+  } else {
+    UP(rowmap, rowmap)
+  }
 #undef UP
   // twiddles (host, double precision): x, y, z tables
   if (!rc) {
@@ -714,9 +758,11 @@ static int sum_energy_slots(const jrg_plan* P, double* slots, double* energies, 
 }
 
 // density of the band-major coefficients held in workspace slot c (qpart:
-// the charge partials of ChargeFix, or null)
+// the charge partials of ChargeFix, or null).  need: weights of the bands whose
+// planes a later adjoint pass reads (a superset of the occupied ones); the
+// column kernels leave out bands of weight zero.
 template <typename R>
-static int density_from_c(const jrg_plan* P, const double* occ, void* ws, void* rho_out,
+static int density_from_c(const jrg_plan* P, const double* occ, const double* need, void* ws, void* rho_out,
                           cudaStream_t st, double* qpart = nullptr) {
   using C = C_t<R>;
   const Workspace& w = P->ws;
@@ -728,7 +774,7 @@ static int density_from_c(const jrg_plan* P, const double* occ, void* ws, void* 
     {
       PHASE(PH_PLANE_INV);
       if ((rc = launch_plane_inv_sphere<R>(P, (C*)wsp(ws, w.c) + (size_t)k0 * P->nb * P->ng, wsp(ws, w.t),
-                                           n * P->nb, st)))
+                                           n * P->nb, need + (size_t)k0 * P->nb, st)))
         return rc;
     }
     {
@@ -799,17 +845,20 @@ static int grid_phase(const jrg_plan* P, const double* occ, double* slots, void*
 // buffers t_in / t_out (block k0 first), with the potential of each block's
 // spin (vr: [ns][grid]); one launch per spin.
 template <typename R>
-static int apply_v_blocks(const jrg_plan* P, void* t_in, void* t_out, const void* vr, int k0, int n,
-                          cudaStream_t st) {
+static int apply_v_blocks(const jrg_plan* P, void* t_in, void* t_out, const void* vr, const double* need,
+                          int k0, int n, cudaStream_t st) {
   using C = C_t<R>;
-  const size_t per_block = (size_t)P->nb * P->nact * P->ny * P->nz;   // plane elements of one block
+  // plane-buffer elements of one block as the inverse pass left them
+  const size_t per_block = (size_t)P->nb * (cols::active(P) ? (size_t)P->nx * P->tpitch
+                                                            : (size_t)P->nact * P->ny * P->nz);
   int rc;
   for (int b = k0; b < k0 + n;) {
     const int s = b / P->nk;
     const int e = std::min(k0 + n, (s + 1) * P->nk);
     const size_t off = (size_t)(b - k0) * per_block;
     if ((rc = launch_line_apply_v<R>(P, (C*)t_in + off, (C*)t_out + off,
-                                     (const R*)vr + (size_t)s * P->ngrid, (e - b) * P->nb, P->nb, st)))
+                                     (const R*)vr + (size_t)s * P->ngrid, (e - b) * P->nb, P->nb,
+                                     need + (size_t)b * P->nb, st)))
       return rc;
     b = e;
   }
@@ -826,6 +875,9 @@ static int energy_grad_impl(const jrg_plan* P, const void* w_re, const void* w_i
   const int nbt = nsk * P->nb;
   const double N = (double)P->ngrid;
   int rc;
+  // weights of g_C: with band energies requested, g_C = H c of every band; else
+  // an empty band has no gradient
+  const double* need = band_e ? P->d_ones : occ;
   JRG_CUDA(cudaMemsetAsync(wsp(ws, w.flags), 0, 64, st));
   int kin_blocks = 0;
   if ((rc = orthonormalise<R>(P, w_re, w_im, ws, st, kRotBand, nullptr, &kin_blocks))) return rc;
@@ -849,8 +901,8 @@ static int energy_grad_impl(const jrg_plan* P, const void* w_re, const void* w_i
                                        (float*)wsp(ws, w.lut), st)))
       return rc;
   }
-  if ((rc = nl_forward<R>(P, ws, 0, nsk, occ, band_e ? P->d_ones : occ, st))) return rc;
-  if ((rc = density_from_c<R>(P, occ, ws, wsp(ws, w.rho), st, (double*)wsp(ws, w.rho_q)))) return rc;
+  if ((rc = nl_forward<R>(P, ws, 0, nsk, occ, need, st))) return rc;
+  if ((rc = density_from_c<R>(P, occ, need, ws, wsp(ws, w.rho), st, (double*)wsp(ws, w.rho_q)))) return rc;
   {
     PHASE(PH_GRID_TERMS);
     if ((rc = grid_phase<R>(P, occ, slots, ws, st))) return rc;
@@ -866,18 +918,20 @@ static int energy_grad_impl(const jrg_plan* P, const void* w_re, const void* w_i
     const size_t co = (size_t)k0 * P->nb * P->ng;
     if (P->kchunk < nsk) {
       PHASE(PH_PLANE_INV);
-      if ((rc = launch_plane_inv_sphere<R>(P, (C*)wsp(ws, w.c) + co, wsp(ws, w.t), n * P->nb, st))) return rc;
+      if ((rc = launch_plane_inv_sphere<R>(P, (C*)wsp(ws, w.c) + co, wsp(ws, w.t), n * P->nb,
+                                           need + (size_t)k0 * P->nb, st)))
+        return rc;
     }
     {
       PHASE(PH_LINE_APPLY_V);
-      if ((rc = apply_v_blocks<R>(P, wsp(ws, w.t), wsp(ws, w.u), wsp(ws, w.vr), k0, n, st))) return rc;
+      if ((rc = apply_v_blocks<R>(P, wsp(ws, w.t), wsp(ws, w.u), wsp(ws, w.vr), need, k0, n, st))) return rc;
     }
     {
       // with band energies requested, g_C = H c unweighted; the occupations
       // are folded into the small adjoint matrices below
       PHASE(PH_PLANE_FWD);
       if ((rc = launch_plane_fwd_sphere<R>(P, wsp(ws, w.u), (C*)wsp(ws, w.c) + co, (C*)wsp(ws, w.gc) + co,
-                                           band_e ? P->d_ones : occ, k0 * P->nb, n * P->nb, 1.0 / N, st)))
+                                           need, k0 * P->nb, n * P->nb, 1.0 / N, st)))
         return rc;
     }
   }
@@ -934,12 +988,13 @@ static int band_trace_impl(const jrg_plan* P, const void* w_re, const void* w_im
     const size_t co = (size_t)k0 * P->nb * P->ng;
     {
       PHASE(PH_PLANE_INV);
-      if ((rc = launch_plane_inv_sphere<R>(P, (C_t<R>*)wsp(ws, w.c) + co, wsp(ws, w.t), n * P->nb, st)))
+      if ((rc = launch_plane_inv_sphere<R>(P, (C_t<R>*)wsp(ws, w.c) + co, wsp(ws, w.t), n * P->nb,
+                                           wts + (size_t)k0 * P->nb, st)))
         return rc;
     }
     {
       PHASE(PH_LINE_APPLY_V);
-      if ((rc = apply_v_blocks<R>(P, wsp(ws, w.t), wsp(ws, w.u), v_eff, k0, n, st))) return rc;
+      if ((rc = apply_v_blocks<R>(P, wsp(ws, w.t), wsp(ws, w.u), v_eff, wts, k0, n, st))) return rc;
     }
     {
       PHASE(PH_PLANE_FWD);
@@ -1011,7 +1066,8 @@ static int phase_forward_range(const jrg_plan* P, const void* w_re, const void* 
   if (kb < 0) return -kb;
   if (kb == 0) return fail(JRG_ERR_UNSUPPORTED, "pipelined path needs the fused kinetic rotation");
   if ((rc = nl_forward<R>(P, ws, k0, n, occ, occ, st))) return rc;
-  if ((rc = launch_plane_inv_sphere<R>(P, (C*)wsp(ws, w.c) + co, (C*)wsp(ws, w.t) + to, n * P->nb, st)))
+  if ((rc = launch_plane_inv_sphere<R>(P, (C*)wsp(ws, w.c) + co, (C*)wsp(ws, w.t) + to, n * P->nb,
+                                       occ + (size_t)k0 * P->nb, st)))
     return rc;
   return launch_line_density<R>(P, (C*)wsp(ws, w.t) + to, (R*)wsp(ws, w.rho_part) + (size_t)k0 * P->ngrid,
                                 occ, 1.0 / P->vol, k0 * P->nb, n * P->nb, P->nb,
@@ -1036,7 +1092,7 @@ static int phase_adjoint_range(const jrg_plan* P, const double* occ, void* g_re,
   C* c = (C*)wsp(ws, w.c) + co;
   C* gc = (C*)wsp(ws, w.gc) + co;
   int rc;
-  if ((rc = apply_v_blocks<R>(P, t, t, wsp(ws, w.vr), k0, n, st))) return rc;
+  if ((rc = apply_v_blocks<R>(P, t, t, wsp(ws, w.vr), occ, k0, n, st))) return rc;
   if ((rc = launch_plane_fwd_sphere<R>(P, t, c, gc, occ, k0 * P->nb, n * P->nb, 1.0 / N, st))) return rc;
   if ((rc = nl_adjoint<R>(P, ws, k0, n, st))) return rc;
   if ((rc = launch_gram<R>(kBand, c, nullptr, kBand, gc, nullptr,
@@ -1145,7 +1201,7 @@ static int density_entry(const jrg_plan* P, const void* coeff, const double* occ
   const int nsk = P->ns * P->nk;
   int rc = launch_pack_params<R>(coeff, nullptr, wsp(ws, P->ws.c), nsk, P->ng, P->nb, true, st);
   if (rc) return rc;
-  return density_from_c<R>(P, occ, ws, rho, st);
+  return density_from_c<R>(P, occ, occ, ws, rho, st);
 }
 
 template <typename R>

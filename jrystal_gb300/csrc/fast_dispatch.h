@@ -21,4 +21,13 @@ template <typename R>
 int dispatch_dense(const FftAxis* ax, const C_t<R>* tw, int batch, int dir, bool real_in,
                    const void* in, C_t<R>* scratch, C_t<R>* out, double scale, cudaStream_t st);
 }  // namespace fast
+namespace cols {
+// column-first kernels of k_fft_cols.cu (same return convention); used when
+// active(P), for every operation of a call
+template <typename R> int dispatch(const jrg_plan* P, int op, const fast::Args& a, cudaStream_t st);
+// whether the column-first kernels take the plan's grid (pruned: the plane-first
+// ones leave out the known zeros of all axes)
+bool covers(int prec, int nx, int ny, int nz, int nb, bool colwin, bool pruned);
+bool active(const jrg_plan* P);
+}  // namespace cols
 }  // namespace jrg

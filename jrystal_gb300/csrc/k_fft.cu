@@ -300,11 +300,11 @@ template <typename K> static int set_smem(K kernel, size_t bytes) {
 
 template <typename R>
 int launch_plane_inv_sphere(const jrg_plan* P, const void* coef, void* planes, int nbands,
-                            cudaStream_t st) {
+                            const double* need, cudaStream_t st) {
   using C = C_t<R>;
   {
-    fast::Args a{coef, planes, nullptr, nullptr, 0.0, 0, nbands, 1};
-    const int f = fast::dispatch<R>(P, fast::OP_PLANE_INV, a, st);
+    fast::Args a{coef, planes, nullptr, need, 0.0, 0, nbands, 1};
+    const int f = cols::active(P) ? cols::dispatch<R>(P, fast::OP_PLANE_INV, a, st) : fast::dispatch<R>(P, fast::OP_PLANE_INV, a, st);
     if (f < 0) return -f;
     if (f > 0) return JRG_OK;
   }
@@ -328,7 +328,7 @@ int launch_line_density(const jrg_plan* P, const void* planes, void* rho_part, c
   using C = C_t<R>;
   {
     fast::Args a{planes, rho_part, nullptr, wband, wscale, band0, nbands, bands_per_group, gscale};
-    const int f = fast::dispatch<R>(P, fast::OP_LINE_DENSITY, a, st);
+    const int f = cols::active(P) ? cols::dispatch<R>(P, fast::OP_LINE_DENSITY, a, st) : fast::dispatch<R>(P, fast::OP_LINE_DENSITY, a, st);
     if (f < 0) return -f;
     if (f > 0) return JRG_OK;
   }
@@ -347,11 +347,11 @@ int launch_line_density(const jrg_plan* P, const void* planes, void* rho_part, c
 
 template <typename R>
 int launch_line_apply_v(const jrg_plan* P, const void* planes_in, void* planes_out, const void* vr,
-                        int nbands, int bands_per_group, cudaStream_t st) {
+                        int nbands, int bands_per_group, const double* need, cudaStream_t st) {
   using C = C_t<R>;
   if (planes_in == planes_out) {   // the fast kernel works in place
-    fast::Args a{planes_in, planes_out, vr, nullptr, 0.0, 0, nbands, bands_per_group};
-    const int f = fast::dispatch<R>(P, fast::OP_LINE_APPLY_V, a, st);
+    fast::Args a{planes_in, planes_out, vr, need, 0.0, 0, nbands, bands_per_group};
+    const int f = cols::active(P) ? cols::dispatch<R>(P, fast::OP_LINE_APPLY_V, a, st) : fast::dispatch<R>(P, fast::OP_LINE_APPLY_V, a, st);
     if (f < 0) return -f;
     if (f > 0) return JRG_OK;
   }
@@ -376,7 +376,7 @@ int launch_plane_fwd_sphere(const jrg_plan* P, const void* planes, const void* c
   using C = C_t<R>;
   {
     fast::Args a{planes, gcoef, coef, wband, scale, band0, nbands, 1};
-    const int f = fast::dispatch<R>(P, fast::OP_PLANE_FWD, a, st);
+    const int f = cols::active(P) ? cols::dispatch<R>(P, fast::OP_PLANE_FWD, a, st) : fast::dispatch<R>(P, fast::OP_PLANE_FWD, a, st);
     if (f < 0) return -f;
     if (f > 0) return JRG_OK;
   }
@@ -440,11 +440,12 @@ int launch_fft3d_dense(const FftAxis* ax, const C_t<R>* tw, int batch, int dir, 
 }
 
 #define JRG_INST(R)                                                                              \
-  template int launch_plane_inv_sphere<R>(const jrg_plan*, const void*, void*, int, cudaStream_t); \
+  template int launch_plane_inv_sphere<R>(const jrg_plan*, const void*, void*, int, const double*,  \
+                                          cudaStream_t);                                         \
   template int launch_line_density<R>(const jrg_plan*, const void*, void*, const double*, double, \
                                       int, int, int, double*, cudaStream_t);                     \
   template int launch_line_apply_v<R>(const jrg_plan*, const void*, void*, const void*, int, int,   \
-                                      cudaStream_t);                                             \
+                                      const double*, cudaStream_t);                              \
   template int launch_plane_fwd_sphere<R>(const jrg_plan*, const void*, const void*, void*,        \
                                           const double*, int, int, double, cudaStream_t);        \
   template int launch_fft3d_dense<R>(const FftAxis*, const C_t<R>*, int, int, bool, const void*,   \

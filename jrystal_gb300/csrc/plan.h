@@ -65,6 +65,8 @@ struct PlanTables {
   double* ginv = nullptr;     // [ngrid] 4 pi / |G|^2, 0 at G = 0
   double* gvec = nullptr;     // [ngrid][3] cartesian G vectors
   void* proj = nullptr;       // [nk][nproj][ng] complex beta-projector table (precision R)
+  int* xmap = nullptr;        // column transforms: [window x][ncol] sphere index, or -1
+  short* col_of = nullptr;    // [window y][window z] column of T, or -1
 };
 
 // Per-phase CUDA-event timing of the fused entry points (optional).
@@ -122,6 +124,12 @@ struct jrg_plan {
   // at or above 3N/4: the x (y, z) transforms skip the known zeros
   bool xprune = false;
   bool yzprune = false;
+  // column-first transforms (k_fft_cols.cu): T[band][x][tpitch] over the ncol
+  // (y, z) columns that the sphere touches; colwin: every active index of all
+  // axes lies in the alias-free window |i| < N/4
+  bool cols = false;
+  bool colwin = false;
+  int ncol = 0, tpitch = 0;
   double cell[9], recip[9], vol;
   std::vector<double> pos, charge, kpts;
   int xc;
