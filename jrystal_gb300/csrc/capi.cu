@@ -18,6 +18,8 @@ template <typename R> int launch_line_density(const jrg_plan*, const void*, void
 template <typename R> int launch_line_apply_v(const jrg_plan*, const void*, void*, const void*, int, int, const double*, cudaStream_t);
 template <typename R> int launch_plane_fwd_sphere(const jrg_plan*, const void*, const void*, void*, const double*, int, int, double, cudaStream_t);
 template <typename R> int launch_fft3d_dense(const FftAxis*, const C_t<R>*, int, int, bool, const void*, C_t<R>*, C_t<R>*, double, cudaStream_t);
+template <typename R> int launch_hartree(const jrg_plan*, const void*, C_t<R>*, C_t<R>*, double*, int, double, double, const ChargeFix&, cudaStream_t);
+template <typename R> int launch_adam_pair(const AdamArgs&, size_t, const void*, const void*, long long, cudaStream_t);
 template <typename R> int launch_pack_params(const void*, const void*, void*, int, int, int, bool, cudaStream_t);
 template <typename R> int launch_unpack(const void*, void*, void*, void*, int, int, int, double, cudaStream_t);
 template <typename R> int launch_gram(int, const void*, const void*, int, const void*, const void*, double2*, double2*, int, int, int, int, cudaStream_t, int* = nullptr, bool = false);
@@ -255,6 +257,8 @@ int jrg_plan_destroy(jrg_plan* P) {
   if (P->fork_ev) cudaEventDestroy(P->fork_ev);
   if (P->join_ev) cudaEventDestroy(P->join_ev);
   if (P->side) cudaStreamDestroy(P->side);
+  if (P->aux_ev) cudaEventDestroy(P->aux_ev);
+  if (P->aux) cudaStreamDestroy(P->aux);
   if (P->prof) {
     for (cudaEvent_t e : P->prof->ev) cudaEventDestroy(e);
     delete P->prof;
@@ -508,6 +512,8 @@ int jrg_plan_create(const jrg_plan_desc* d, jrg_plan** out) {
     cudaError_t e = cudaStreamCreateWithFlags(&P->side, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&P->fork_ev, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&P->join_ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&P->aux, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&P->aux_ev, cudaEventDisableTiming);
     if (e != cudaSuccess) rc = cuda_fail(e, "stream/event creation");
   }
   if (!rc) {
@@ -809,6 +815,8 @@ static int grid_phase(const jrg_plan* P, const double* occ, double* slots, void*
   double* q = (double*)wsp(ws, w.rho_q);
   ChargeFix cf;
   cf.qpart = q;
+  const int per16 = 16 / rsize(P->prec);   // as launch_reduce_density
+  cf.nq = q_parts(P->ns * P->ngrid, P->ngrid % per16 == 0 ? per16 : 1);
   cf.occ = occ;
   cf.nocc = nbt;
   cf.dv = P->vol / N;
@@ -823,14 +831,21 @@ static int grid_phase(const jrg_plan* P, const double* occ, double* slots, void*
     if ((rc = launch_spin_total<R>(rho, tot, P->ngrid, st))) return rc;
     rho_t = tot;
   }
-  if ((rc = launch_fft3d_dense<R>(P->ax, tw, 1, -1, true, rho_t, scratch, rhog, 1.0, st))) return rc;
   const bool gga = (P->xc & kXcGga) != 0;
-  if (gga && (rc = gga_gradients<R>(P, rhog, ws, st))) return rc;
-  // Hartree energy and V_H(G) (in place)
-  if ((rc = launch_recip_terms<R>(rhog, P->d.ginv, rhog, slot_h, kRecipBlocks, P->ngrid, P->vol / (N * N),
-                                  cf, st)))
-    return rc;
-  if ((rc = launch_fft3d_dense<R>(P->ax, tw, 1, +1, false, rhog, scratch, rhog, 1.0 / N, st))) return rc;
+  int fused = 0;
+  if (!gga) {
+    fused = launch_hartree<R>(P, rho_t, scratch, rhog, slot_h, kRecipBlocks, P->vol / (N * N), 1.0 / N, cf, st);
+    if (fused < 0) return -fused;
+  }
+  if (!fused) {
+    // rho(G) itself (the gradients of PBE), then Hartree energy and V_H(G) in place
+    if ((rc = launch_fft3d_dense<R>(P->ax, tw, 1, -1, true, rho_t, scratch, rhog, 1.0, st))) return rc;
+    if (gga && (rc = gga_gradients<R>(P, rhog, ws, st))) return rc;
+    if ((rc = launch_recip_terms<R>(rhog, P->d.ginv, rhog, slot_h, kRecipBlocks, P->ngrid, P->vol / (N * N),
+                                    cf, st)))
+      return rc;
+    if ((rc = launch_fft3d_dense<R>(P->ax, tw, 1, +1, false, rhog, scratch, rhog, 1.0 / N, st))) return rc;
+  }
   if (gga)
     return gga_potential<R>(P, rho, rhog, 1.0, wsp(ws, w.vr), slot_x, 0, ws, st, cf.scale, P->d.vext_r,
                             slot_e);
@@ -1114,15 +1129,7 @@ static int phase_adjoint_range(const jrg_plan* P, const double* occ, void* g_re,
                              n, P->ng, P->nb, 2.0, wsp(ws, w.rot_scratch), st, kTriLower)))
     return rc;
   if (!adam) return JRG_OK;
-  for (int part = 0; part < 2; ++part) {
-    const float* sc = adam->scale[part] ? adam->scale[part] + po : nullptr;
-    if ((rc = launch_adam<R>(reinterpret_cast<R*>(adam->p[part]) + po, part ? gi : gr,
-                             reinterpret_cast<R*>(adam->m[part]) + po,
-                             reinterpret_cast<R*>(adam->v[part]) + po, sc, (long long)cnt, adam->lr,
-                             adam->b1, adam->b2, adam->c1, adam->c2, adam->eps, st, adam->guard)))
-      return rc;
-  }
-  return JRG_OK;
+  return launch_adam_pair<R>(*adam, po, gr, gi, (long long)cnt, st);
 }
 
 static bool g_pipeline = true;   // two-way k-point pipeline of jrg_energy_grad
@@ -1161,10 +1168,17 @@ static int energy_grad_pipelined(const jrg_plan* P, const void* w_re, const void
   if ((rc = phase_forward_range<R>(P, w_re, w_im, occ, ws, ka, kb, P->side))) return rc;
   if ((rc = join())) return rc;
   double* slots = (double*)wsp(ws, w.epart);
-  if ((rc = launch_kin_reduce(P->prec, wsp(ws, w.kin_part), (P->ng + 255) / 256, P->nb, nbt, occ, slots,
-                              (double*)wsp(ws, w.ekin), st)))
-    return rc;
-  if (adam && adam->mlp_w32 &&
+  // The kinetic reduction and the energy sums feed only the energies (and the
+  // learned scales): with a gradient they run on the plan's third stream beside
+  // the adjoint halves, 13 us off the chain of a small cell's step.
+  const bool grad = adam || g_re || g_im;
+  const bool learned = adam && adam->mlp_w32;
+  auto kinetic = [&](cudaStream_t s) {
+    return launch_kin_reduce(P->prec, wsp(ws, w.kin_part), (P->ng + 255) / 256, P->nb, nbt, occ, slots,
+                             (double*)wsp(ws, w.ekin), s);
+  };
+  if ((learned || !grad) && (rc = kinetic(st))) return rc;
+  if (learned &&
       (rc = launch_precond_scale_lut(adam->mlp_w32, adam->mlp_wb, P->d.tk, P->d.tkf, P->tk_max,
                                      (const double*)wsp(ws, w.ekin), occ, P->nk, P->ng, P->nb, nbt,
                                      (long long)nbt * P->ng, adam->t_frac, adam->smax, adam->scale[0],
@@ -1174,15 +1188,18 @@ static int energy_grad_pipelined(const jrg_plan* P, const void* w_re, const void
                                      (const double*)wsp(ws, w.rho_scale), (double*)wsp(ws, w.rho_q), st)))
     return rc;
   if ((rc = grid_phase<R>(P, occ, slots, ws, st))) return rc;
-  // the energy sums feed only the energies output: they run after the adjoint
-  // halves, off the path between the two forks
-  if (!adam && !g_re && !g_im) return sum_energy_slots(P, slots, energies, ws, st);
+  if (!grad) return sum_energy_slots(P, slots, energies, ws, st);
   if (!adam && (!g_re || !g_im)) return fail(JRG_ERR_INVALID, "grad_re and grad_im must both be given");
   if ((rc = fork())) return rc;
-  if ((rc = phase_adjoint_range<R>(P, occ, g_re, g_im, ws, 0, ka, st, adam))) return rc;
-  if ((rc = phase_adjoint_range<R>(P, occ, g_re, g_im, ws, ka, kb, P->side, adam))) return rc;
-  if ((rc = join())) return rc;
-  return sum_energy_slots(P, slots, energies, ws, st);
+  JRG_CUDA(cudaStreamWaitEvent(P->aux, P->fork_ev, 0));
+  rc = learned ? JRG_OK : kinetic(P->aux);
+  if (!rc) rc = sum_energy_slots(P, slots, energies, ws, P->aux);
+  JRG_CUDA(cudaEventRecord(P->aux_ev, P->aux));
+  if (!rc) rc = phase_adjoint_range<R>(P, occ, g_re, g_im, ws, 0, ka, st, adam);
+  if (!rc) rc = phase_adjoint_range<R>(P, occ, g_re, g_im, ws, ka, kb, P->side, adam);
+  const int joined = join();
+  JRG_CUDA(cudaStreamWaitEvent(st, P->aux_ev, 0));
+  return rc ? rc : joined;
 }
 
 template <typename R>

@@ -20,6 +20,10 @@ template <typename R> int dispatch(const jrg_plan* P, int op, const Args& a, cud
 template <typename R>
 int dispatch_dense(const FftAxis* ax, const C_t<R>* tw, int batch, int dir, bool real_in,
                    const void* in, C_t<R>* scratch, C_t<R>* out, double scale, cudaStream_t st);
+// V_H(r) and the E_H partials of a density, cubic grids (same return convention)
+template <typename R>
+int dispatch_hartree(const jrg_plan* P, const void* rho, C_t<R>* mid, C_t<R>* rhog, double* slot_h, int nslots,
+                     double pref, double inv_n, const ChargeFix& cf, cudaStream_t st);
 }  // namespace fast
 namespace cols {
 // column-first kernels of k_fft_cols.cu (same return convention); used when

@@ -12,6 +12,7 @@
 // only y rows that hold sphere points are transformed where the data are
 // known to be zero.  The intermediate between the two kernels holds only the
 // active planes: [band][active plane][y][z].
+#include "charge.cuh"
 #include "fast_dispatch.h"
 #include "plan.h"
 
@@ -283,6 +284,51 @@ __global__ void __launch_bounds__(kLineThreads) k_line_dense(const C_t<R>* __res
   }
 }
 
+// the Hartree line pass of k_fft_fast.cu's k_line_hartree on any grid
+template <typename R>
+__global__ void __launch_bounds__(kLineThreads) k_line_hartree(C_t<R>* __restrict__ io,
+                                                               const C_t<R>* __restrict__ tw_x, FftAxis axx, int nx,
+                                                               int ny, int nz, const double* __restrict__ ginv,
+                                                               double* __restrict__ slot_h, int nslots, double pref,
+                                                               double inv_n, ChargeFix cf) {
+  using C = C_t<R>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double red[32];
+  const int slab = nx * nz;
+  C* twx = reinterpret_cast<C*>(smem_raw);
+  C* A = twx + nx;
+  C* B = A + slab;
+  const int y = blockIdx.x;
+  for (int i = threadIdx.x; i < nx; i += blockDim.x) twx[i] = tw_x[i];
+  for (int i = threadIdx.x; i < slab; i += blockDim.x) {
+    const int x = i / nz, z = i - x * nz;
+    A[i] = io[((size_t)x * ny + y) * nz + z];
+  }
+  const double s = charge_scale(cf, red);
+  if (cf.scale && blockIdx.x == 0 && threadIdx.x == 0) *cf.scale = s;
+  __syncthreads();
+  C* res = fft_lines<-1>(A, B, twx, axx, nz, nz, 1, nullptr, true);
+  double eh = 0.0;
+  for (int i = threadIdx.x; i < slab; i += blockDim.x) {
+    const int x = i / nz, z = i - x * nz;
+    const double gi = ginv[((size_t)x * ny + y) * nz + z];
+    const double rx = res[i].x, ry = res[i].y, t = s * gi * inv_n;
+    eh += 0.5 * gi * (rx * rx + ry * ry);
+    res[i].x = (R)(t * rx);
+    res[i].y = (R)(t * ry);
+  }
+  __syncthreads();
+  res = fft_lines<+1>(res, res == A ? B : A, twx, axx, nz, nz, 1, nullptr, true);
+  for (int i = threadIdx.x; i < slab; i += blockDim.x) {
+    const int x = i / nz, z = i - x * nz;
+    io[((size_t)x * ny + y) * nz + z] = res[i];
+  }
+  eh = block_sum(eh, red);
+  if (threadIdx.x == 0) slot_h[blockIdx.x] = eh * pref * s * s;
+  if (blockIdx.x == 0)
+    for (int i = gridDim.x + threadIdx.x; i < nslots; i += blockDim.x) slot_h[i] = 0.0;
+}
+
 // ------------------------------------------------------------------------
 // host launchers
 // ------------------------------------------------------------------------
@@ -439,6 +485,35 @@ int launch_fft3d_dense(const FftAxis* ax, const C_t<R>* tw, int batch, int dir, 
   return JRG_OK;
 }
 
+// V_H(r) (complex, in rhog) and the E_H partials of the density rho (see
+// k_line_hartree); mid: a work grid.  1: launched, 0: more rows than slots, < 0: -status
+template <typename R>
+int launch_hartree(const jrg_plan* P, const void* rho, C_t<R>* mid, C_t<R>* rhog, double* slot_h, int nslots,
+                   double pref, double inv_n, const ChargeFix& cf, cudaStream_t st) {
+  using C = C_t<R>;
+  const int f = fast::dispatch_hartree<R>(P, rho, mid, rhog, slot_h, nslots, pref, inv_n, cf, st);
+  if (f) return f;
+  const int nx = P->nx, ny = P->ny, nz = P->nz;
+  if (ny > nslots) return 0;
+  const C* tw = reinterpret_cast<const C*>(P->d.tw);
+  const size_t smp = plane_smem<R>(ny, nz, 0), sml = line_smem<R>(nx, nz, 0, 0);
+  int rc;
+  if ((rc = set_smem(k_plane_dense<R, -1, true>, smp))) return -rc;
+  if ((rc = set_smem(k_plane_dense<R, +1, false>, smp))) return -rc;
+  if ((rc = set_smem(k_line_hartree<R>, sml))) return -rc;
+  k_plane_dense<R, -1, true><<<dim3(nx, 1), 256, smp, st>>>(rho, mid, tw + nx, tw + nx + ny, P->ax[1], P->ax[2], nx,
+                                                             ny, nz);
+  count_launch();
+  k_line_hartree<R><<<ny, kLineThreads, sml, st>>>(mid, tw, P->ax[0], nx, ny, nz, P->d.ginv, slot_h, nslots, pref,
+                                                   inv_n, cf);
+  count_launch();
+  k_plane_dense<R, +1, false><<<dim3(nx, 1), 256, smp, st>>>(mid, rhog, tw + nx, tw + nx + ny, P->ax[1], P->ax[2], nx,
+                                                              ny, nz);
+  count_launch();
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 1 : -cuda_fail(e, "k_line_hartree");
+}
+
 #define JRG_INST(R)                                                                              \
   template int launch_plane_inv_sphere<R>(const jrg_plan*, const void*, void*, int, const double*,  \
                                           cudaStream_t);                                         \
@@ -449,7 +524,9 @@ int launch_fft3d_dense(const FftAxis* ax, const C_t<R>* tw, int batch, int dir, 
   template int launch_plane_fwd_sphere<R>(const jrg_plan*, const void*, const void*, void*,        \
                                           const double*, int, int, double, cudaStream_t);        \
   template int launch_fft3d_dense<R>(const FftAxis*, const C_t<R>*, int, int, bool, const void*,   \
-                                     C_t<R>*, C_t<R>*, double, cudaStream_t);
+                                     C_t<R>*, C_t<R>*, double, cudaStream_t);                    \
+  template int launch_hartree<R>(const jrg_plan*, const void*, C_t<R>*, C_t<R>*, double*, int, double, \
+                                 double, const ChargeFix&, cudaStream_t);
 JRG_INST(float)
 JRG_INST(double)
 

@@ -10,6 +10,7 @@
 // consecutive lines: consecutive z in global memory, consecutive addresses
 // in the exchange buffers, and an odd row pitch (N + 1) in the [z][y] plane
 // buffer keeps the column accesses free of bank conflicts.
+#include "charge.cuh"
 #include "fast_dispatch.h"
 #include "fft_reg.cuh"
 #include <cstdlib>
@@ -645,6 +646,63 @@ __global__ void __launch_bounds__(threads_for<N>()) k_line_dense(const C_t<R>* _
   for (int j = 0; j < N1; ++j) out[base + (size_t)(N2 * j + j2) * (N * N)] = cscale(v[j], sc);
 }
 
+// x forward, Hartree term, x inverse of one (y, half of z) of a density
+// transformed in y and z, in place (the Hartree term of k_recip_terms between two
+// dense line passes): V_H(G) = inv_n s ginv rho(G), E_H partials of the CTA in
+// slot_h.  One kernel instead of three between the forks of a step, where their
+// launches and latencies are exposed: line 4.3 + term 12 + line 4.6 us at 24^3.
+template <int N> __host__ __device__ constexpr int hartree_lines() { return N % 2 == 0 ? N / 2 : N; }
+template <int N> __host__ __device__ constexpr int hartree_threads() { return (hartree_lines<N>() * Split<N>::N2 + 31) / 32 * 32; }
+template <typename R, int N>
+__global__ void __launch_bounds__(hartree_threads<N>()) k_line_hartree(
+    C_t<R>* __restrict__ io, const C_t<R>* __restrict__ tw_g, const double* __restrict__ ginv,
+    double* __restrict__ slot_h, int nslots, double pref, double inv_n, ChargeFix cf) {
+  using C = C_t<R>;
+  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2, L = hartree_lines<N>();
+  __shared__ C tw[N];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double red[32];
+  C* ex = reinterpret_cast<C*>(smem_raw);   // [N][L]
+  const int tid = threadIdx.x, y = blockIdx.x;
+  const bool act = tid < L * N2;
+  const int zl = act ? tid % L : 0, j2 = act ? tid / L : 0, z = blockIdx.y * L + zl;
+  C* line = io + (size_t)y * N + z;
+  C v[N1];
+#pragma unroll
+  for (int j1 = 0; j1 < N1; ++j1) v[j1] = act ? line[(size_t)(N2 * j1 + j2) * (N * N)] : czero<C>();
+  for (int i = tid; i < N; i += blockDim.x) tw[i] = tw_g[i];
+  const double s = charge_scale(cf, red);
+  const int cta = blockIdx.x * gridDim.y + blockIdx.y, nctas = gridDim.x * gridDim.y;
+  if (cf.scale && cta == 0 && tid == 0) *cf.scale = s;
+  __syncthreads();
+  if (act) reg::line_step_a<N, -1>(v, tw, j2, ex, L, zl);
+  __syncthreads();
+  double eh = 0.0;
+  if (act) {
+    reg::line_step_b<N, -1>(v, j2, ex, L, zl);
+#pragma unroll
+    for (int j = 0; j < N1; ++j) {
+      const double gi = ginv[((size_t)(N2 * j + j2) * N + y) * N + z];
+      const double rx = v[j].x, ry = v[j].y, t = s * gi * inv_n;
+      eh += 0.5 * gi * (rx * rx + ry * ry);
+      v[j].x = (R)(t * rx);
+      v[j].y = (R)(t * ry);
+    }
+  }
+  __syncthreads();
+  if (act) reg::line_step_a<N, +1>(v, tw, j2, ex, L, zl);
+  __syncthreads();
+  if (act) {
+    reg::line_step_b<N, +1>(v, j2, ex, L, zl);
+#pragma unroll
+    for (int j = 0; j < N1; ++j) line[(size_t)(N2 * j + j2) * (N * N)] = v[j];
+  }
+  eh = block_sum(eh, red);
+  if (tid == 0) slot_h[cta] = eh * pref * s * s;
+  if (cta == 0)
+    for (int i = nctas + tid; i < nslots; i += blockDim.x) slot_h[i] = 0.0;
+}
+
 // ------------------------------------------------------------------------
 // dispatch: returns 1 when a fast kernel was launched, 0 when the grid is not
 // covered (the caller then uses the generic kernels), <0 on a launch error.
@@ -923,6 +981,45 @@ template int dispatch_dense<float>(const FftAxis*, const C_t<float>*, int, int, 
                                    C_t<float>*, C_t<float>*, double, cudaStream_t);
 template int dispatch_dense<double>(const FftAxis*, const C_t<double>*, int, int, bool, const void*,
                                     C_t<double>*, C_t<double>*, double, cudaStream_t);
+
+// V_H(r) (complex, in rhog) of the density rho: y and z forward, the Hartree line
+// pass, y and z inverse; mid: a work grid
+template <typename R, int N>
+static int hartree_run(const C_t<R>* tw, const void* rho, C_t<R>* mid, C_t<R>* rhog, const double* ginv,
+                       double* slot_h, int nslots, double pref, double inv_n, const ChargeFix& cf, cudaStream_t st) {
+  using C = C_t<R>;
+  constexpr int T = threads_for<N>(), L = hartree_lines<N>();
+  const size_t smp = sizeof(C) * (size_t)(N + N * (N + 1) + N * N), sml = sizeof(C) * (size_t)N * L;
+  if (N * (N / L) > nslots) return 0;
+  int rc;
+  if ((rc = prep(k_plane_dense<R, N, -1, true>, smp)) <= 0) return rc;
+  if ((rc = prep(k_plane_dense<R, N, +1, false>, smp)) <= 0) return rc;
+  if ((rc = prep(k_line_hartree<R, N>, sml)) <= 0) return rc;
+  k_plane_dense<R, N, -1, true><<<dim3(N, 1), T, smp, st>>>(rho, mid, tw);
+  ::jrg::count_launch();
+  k_line_hartree<R, N><<<dim3(N, N / L), hartree_threads<N>(), sml, st>>>(mid, tw, ginv, slot_h, nslots, pref, inv_n,
+                                                                         cf);
+  ::jrg::count_launch();
+  k_plane_dense<R, N, +1, false><<<dim3(N, 1), T, smp, st>>>(mid, rhog, tw);
+  FAST_LAUNCHED("fast::k_line_hartree");
+}
+
+template <typename R>
+int dispatch_hartree(const jrg_plan* P, const void* rho, C_t<R>* mid, C_t<R>* rhog, double* slot_h, int nslots,
+                     double pref, double inv_n, const ChargeFix& cf, cudaStream_t st) {
+  if (!g_fast_enabled || !(P->nx == P->ny && P->ny == P->nz)) return 0;
+  const C_t<R>* tw = reinterpret_cast<const C_t<R>*>(P->d.tw);
+  switch (P->nx) {
+#define CASE(N) case N: return hartree_run<R, N>(tw, rho, mid, rhog, P->d.ginv, slot_h, nslots, pref, inv_n, cf, st);
+    CASE(16) CASE(24) CASE(27) CASE(32) CASE(36) CASE(48) CASE(64) CASE(96)
+#undef CASE
+    default: return 0;
+  }
+}
+template int dispatch_hartree<float>(const jrg_plan*, const void*, float2*, float2*, double*, int, double, double,
+                                     const ChargeFix&, cudaStream_t);
+template int dispatch_hartree<double>(const jrg_plan*, const void*, double2*, double2*, double*, int, double, double,
+                                      const ChargeFix&, cudaStream_t);
 
 }  // namespace fast
 }  // namespace jrg

@@ -2,6 +2,7 @@
 // external energies, LDA exchange-correlation, potential assembly, kinetic
 // energy on the sphere, energy-slot reduction, geometry tables and Ewald.
 // Energy sums are accumulated in FP64 per block and reduced deterministically.
+#include "charge.cuh"
 #include "plan.h"
 
 namespace jrg {
@@ -9,7 +10,7 @@ namespace jrg {
 // rho[s][i] = sum over the groups g of spin s of gscale[g] part[g][i] (FP64
 // sum; gscale = the group's reference weight over the cell volume); with
 // qpart, block b also stores the FP64 sum of the rho values it wrote
-// (kQParts blocks)
+// (q_parts blocks)
 // FP32 partials are summed in float-float arithmetic (each gscale as hi + lo,
 // exact products by FMA, two-sum accumulation: about 2^-44 relative, with
 // FP32 instructions instead of the GPU's slow FP64 pipe); FP64 partials in
@@ -206,17 +207,6 @@ __global__ void __launch_bounds__(256) k_reduce_density_v(const R* __restrict__ 
 // k_potential, k_potential_pol; their CTA count is the number of energy
 // slots)
 constexpr int kGridThreads = 256;   // 512: k_recip_terms 34 vs 19 us, k_potential 28 vs 19 us (64^3)
-
-// the charge factor s of ChargeFix (every thread of the block gets it)
-__device__ __forceinline__ double charge_scale(const ChargeFix& cf, double* red) {
-  if (!cf.qpart) return 1.0;
-  double a = 0.0, t = 0.0;
-  for (int i = threadIdx.x; i < kQParts; i += blockDim.x) a += cf.qpart[i];
-  for (int i = threadIdx.x; i < cf.nocc; i += blockDim.x) t += cf.occ[i];
-  a = block_sum(a, red) * cf.dv;
-  t = block_sum(t, red);
-  return (a > 0.0 && t > 0.0) ? t / a : 1.0;
-}
 
 // Hartree term of a single (spin-summed) density transform rhog, for the
 // renormalised density s rho (s from ChargeFix; block 0 stores it):
@@ -947,7 +937,7 @@ __global__ void k_ewald_finish(const double* __restrict__ slots, int nslots, con
 // ------------------------------------------------------------------------
 
 template <typename R>
-__global__ void k_adam(R* __restrict__ p, const R* __restrict__ g, R* __restrict__ m,
+__device__ __forceinline__ void adam_range(R* __restrict__ p, const R* __restrict__ g, R* __restrict__ m,
                        R* __restrict__ v, const float* __restrict__ scale, long long n, R lr, R b1,
                        R b2, R c1, R c2, R eps, const int* __restrict__ guard,
                        const double* __restrict__ coefs) {
@@ -1043,6 +1033,25 @@ __global__ void k_twiddles(int n, C_t<R>* __restrict__ out) {
   }
 }
 
+template <typename R>
+__global__ void k_adam(R* __restrict__ p, const R* __restrict__ g, R* __restrict__ m, R* __restrict__ v,
+                       const float* __restrict__ scale, long long n, R lr, R b1, R b2, R c1, R c2, R eps,
+                       const int* __restrict__ guard, const double* __restrict__ coefs) {
+  adam_range<R>(p, g, m, v, scale, n, lr, b1, b2, c1, c2, eps, guard, coefs);
+}
+
+// real and imaginary parts in one launch (blockIdx.y): the optimiser step of a
+// small cell is a chain of short kernels, 5 us for each launch of this one
+template <typename R> struct AdamPair {
+  R* p[2]; const R* g[2]; R* m[2]; R* v[2]; const float* scale[2];
+};
+template <typename R>
+__global__ void k_adam_pair(AdamPair<R> a, long long n, R lr, R b1, R b2, R c1, R c2, R eps,
+                            const int* __restrict__ guard) {
+  const int q = blockIdx.y;
+  adam_range<R>(a.p[q], a.g[q], a.m[q], a.v[q], a.scale[q], n, lr, b1, b2, c1, c2, eps, guard, nullptr);
+}
+
 // ------------------------------------------------------------------------
 // launch helpers
 // ------------------------------------------------------------------------
@@ -1058,12 +1067,12 @@ int launch_reduce_density(const void* part, void* rho, int groups_per_spin, int 
                           const double* gscale, double* qpart, cudaStream_t st) {
   constexpr int W = Vec16<R>::n;
   if (ngrid % W == 0 && ((reinterpret_cast<uintptr_t>(part) | reinterpret_cast<uintptr_t>(rho)) & 15) == 0) {
-    k_reduce_density_v<R><<<kQParts, 256, 0, st>>>(reinterpret_cast<const R*>(part), reinterpret_cast<R*>(rho),
+    k_reduce_density_v<R><<<q_parts(ns * ngrid, W), 256, 0, st>>>(reinterpret_cast<const R*>(part), reinterpret_cast<R*>(rho),
                                                    groups_per_spin, ns, ngrid, gscale, qpart);
     JRG_LAUNCH_CHECK("k_reduce_density_v");
     return JRG_OK;
   }
-  k_reduce_density<R><<<kQParts, 256, 0, st>>>(reinterpret_cast<const R*>(part), reinterpret_cast<R*>(rho),
+  k_reduce_density<R><<<q_parts(ns * ngrid, 1), 256, 0, st>>>(reinterpret_cast<const R*>(part), reinterpret_cast<R*>(rho),
                                                groups_per_spin, ns, ngrid, gscale, qpart);
   JRG_LAUNCH_CHECK("k_reduce_density");
   return JRG_OK;
@@ -1241,6 +1250,25 @@ int launch_ewald(const double* cell, const double* gvec, const double* pos, cons
   JRG_LAUNCH_CHECK("k_ewald_finish");
   return JRG_OK;
 }
+
+// Adam of both parts of n elements from offset off (g: the parts' gradients there)
+template <typename R>
+int launch_adam_pair(const AdamArgs& a, size_t off, const void* g0, const void* g1, long long n, cudaStream_t st) {
+  AdamPair<R> q;
+  for (int part = 0; part < 2; ++part) {
+    q.p[part] = reinterpret_cast<R*>(a.p[part]) + off;
+    q.m[part] = reinterpret_cast<R*>(a.m[part]) + off;
+    q.v[part] = reinterpret_cast<R*>(a.v[part]) + off;
+    q.g[part] = reinterpret_cast<const R*>(part ? g1 : g0);
+    q.scale[part] = a.scale[part] ? a.scale[part] + off : nullptr;
+  }
+  k_adam_pair<R><<<dim3(grid_for((n + 3) / 4, 256, 152 * 8), 2), 256, 0, st>>>(q, n, (R)a.lr, (R)a.b1, (R)a.b2, (R)a.c1,
+                                                                    (R)a.c2, (R)a.eps, a.guard);
+  JRG_LAUNCH_CHECK("k_adam_pair");
+  return JRG_OK;
+}
+template int launch_adam_pair<float>(const AdamArgs&, size_t, const void*, const void*, long long, cudaStream_t);
+template int launch_adam_pair<double>(const AdamArgs&, size_t, const void*, const void*, long long, cudaStream_t);
 
 template <typename R>
 int launch_adam(void* p, const void* g, void* m, void* v, const float* scale, long long n, double lr,

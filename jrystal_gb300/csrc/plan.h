@@ -37,9 +37,15 @@ bool factor_axis(int n, FftAxis* ax);
 // in qpart, k_recip_terms forms s = sum occ / (vol/N sum rho) (1 without
 // qpart) and stores it in *scale, and the Hartree, external and xc terms use
 // s rho.
-constexpr int kQParts = 1024;   // CTAs of k_reduce_density, one charge partial each
+constexpr int kQParts = 1024;   // most CTAs of k_reduce_density, one charge partial each
+// its CTAs for n values in 16-byte vectors of w: no more than have work
+inline int q_parts(long long n, int w) {
+  const long long b = (n / w + 255) / 256;
+  return b < 1 ? 1 : (b < kQParts ? (int)b : kQParts);
+}
 struct ChargeFix {
-  const double* qpart = nullptr;  // [kQParts]
+  const double* qpart = nullptr;  // [nq]
+  int nq = 0;
   const double* occ = nullptr;    // [nocc]
   int nocc = 0;
   double dv = 0.0;                // vol / N
@@ -147,5 +153,7 @@ struct jrg_plan {
   double* d_ones = nullptr;   // [S*K*B] ones: unweighted band weights
   cudaStream_t side = nullptr;   // second stream of the two-way k-point pipeline
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
+  cudaStream_t aux = nullptr;    // sums that only the energies need, beside the adjoint halves
+  cudaEvent_t aux_ev = nullptr;
   jrg::Profiler* prof = nullptr;
 };
