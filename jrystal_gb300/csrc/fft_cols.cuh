@@ -203,7 +203,7 @@ template <class Bytes>
 SlabShape slab_shape(int zlines, int ylines, int bands, int regs_threads, Bytes&& bytes) {
   SlabShape best;
   double best_cost = 1e30;
-  for (int t = 64; t <= std::min(zlines > 64 ? 256 : kSlabMost, regs_threads); t += 32) {
+  for (int t = 64; t <= (zlines > 64 ? regs_threads : kSlabMost); t += 32) {
     const int sub = t / zlines;
     if (sub < 1) continue;
     for (int tile = 1; tile <= 24 && tile <= std::max(1, bands); ++tile) {

@@ -9,13 +9,22 @@
 namespace jrg {
 namespace cols {
 
-// 168 registers hold an FP32 line of 64 of the adjoint pass
+// 168 registers hold an FP32 line of 64 of the adjoint pass, or half a line of 96
+// of either pass (density at 96^3: 2.32 ms with 256 threads, 1.46 with 384)
 template <typename R, int N> __host__ __device__ constexpr int cube_apply_threads() {
-  return sizeof(R) == 4 && N <= 64 ? 384 : 256;
+  return sizeof(R) == 4 ? 384 : 256;
+}
+// the z phase of the adjoint pass by pairs of threads (FP64, bound by its
+// arithmetic, gains nothing: 48^3 414 us, by pairs 440)
+template <typename R, int N> __host__ __device__ constexpr bool cube_pairs() {
+  return sizeof(R) == 4 && halves<R, N>();
+}
+template <typename R, int N> __host__ __device__ constexpr int cube_density_threads() {
+  return sizeof(R) == 4 && N > 64 ? 384 : 256;
 }
 
 template <typename R, int N>
-__global__ void __launch_bounds__(kDensityThreads)
+__global__ void __launch_bounds__(cube_density_threads<R, N>())
 k_cube_density(C_t<R>* __restrict__ T, R* __restrict__ rho_part, const double* __restrict__ wband, double wscale,
                int band0, int nband, int bands_per_group, const short* __restrict__ col_of, int tp, int tile, int sub,
                double* __restrict__ gscale) {
@@ -121,7 +130,8 @@ k_cube_apply_v(C_t<R>* __restrict__ T, const R* __restrict__ vr, const double* _
     y_inverse_body<C, N, W>(q);
     __syncthreads();
     prefetch_tile<C>(q.src, list + b0 + tile, min(tile, nl - b0 - tile), tp, q.bstride);
-    z_apply_body<C, N, W>(q, (int)lay.grid, N, PV, sub);
+    if constexpr (cube_pairs<R, N>()) z_apply_pairs<C, N, W>(q, (int)lay.grid, PV, sub);
+    else z_apply_body<C, N, W>(q, (int)lay.grid, N, PV, sub);
     __syncthreads();
     y_forward_body<C, N, W>(q);
     __syncthreads();
@@ -138,7 +148,7 @@ template <typename R, int N> int run_cube(const jrg_plan* P, int op, const fast:
   constexpr int ylines = (halves<R, N>() ? 2 : 1) * win_n<N>();
   int rc;
   if (op == fast::OP_LINE_DENSITY) {
-    const SlabShape s = slab_shape((halves<R, N>() ? 2 : 1) * N, ylines, std::min(a.nbands, bpg), kDensityThreads,
+    const SlabShape s = slab_shape((halves<R, N>() ? 2 : 1) * N, ylines, std::min(a.nbands, bpg), cube_density_threads<R, N>(),
                                    [&](int tile) { return SlabLayout<R>(tile, N, N, 0, bpg, true, false).total; });
     if ((rc = prep((const void*)k_cube_density<R, N>, s.smem)) <= 0) return rc;
     k_cube_density<R, N><<<dim3(N, groups), s.threads, s.smem, st>>>(
@@ -146,7 +156,7 @@ template <typename R, int N> int run_cube(const jrg_plan* P, int op, const fast:
         bpg, P->d.col_of, P->tpitch, s.tile, s.sub, a.gscale);
     return launched("k_cube_density");
   }
-  const SlabShape s = slab_shape(N, ylines, std::min(a.nbands, bpg), cube_apply_threads<R, N>(), [&](int tile) {
+  const SlabShape s = slab_shape((cube_pairs<R, N>() ? 2 : 1) * N, ylines, std::min(a.nbands, bpg), cube_apply_threads<R, N>(), [&](int tile) {
     return SlabLayout<R>(tile, N, N, P->ncol, bpg, false, halves<R, N>()).total;
   });
   if ((rc = prep((const void*)k_cube_apply_v<R, N>, s.smem)) <= 0) return rc;
