@@ -63,39 +63,71 @@ __device__ __forceinline__ void rg_load(const void* __restrict__ a, const void* 
   }
 }
 
-// acc[q][jj] += x[q] * M[row][jj] for the TG G vectors and NJ columns
-template <typename R, int NJ, int TG>
-__device__ __forceinline__ void rg_fma_row(C_t<R> (&acc)[TG][NJ], const C_t<R> (&x)[TG],
-                                           const C_t<R>* __restrict__ mrow) {
-  if constexpr (sizeof(R) == 4) {
+// Accumulators of TG G vectors x NJ columns and acc[q][jj] += x[q] * M[row][jj].
+// FP32: packed over pairs of columns (fma.rn.f32x2: the FP32 pipe's rate at half
+// the issue slots), M staged as (re, re', im, im') of a pair, one 16-byte load.
+// Scalar before: adjoint and Adam 240 us, packed 220 (Si8, 24 bands); 160 bands:
+// forward 1.64 and 1.57 ms, adjoint and Adam 4.55 and 4.47 ms.
+template <typename R, int NJ, int TG> struct RgAcc {
+  C_t<R> v[TG][NJ];
+  __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int jj = 0; jj < NJ; jj += 2) {
-      const float4 m = *reinterpret_cast<const float4*>(mrow + jj);
+    for (int q = 0; q < TG; ++q)
 #pragma unroll
-      for (int q = 0; q < TG; ++q) {
-        acc[q][jj].x = fmaf(x[q].x, m.x, fmaf(-x[q].y, m.y, acc[q][jj].x));
-        acc[q][jj].y = fmaf(x[q].x, m.y, fmaf(x[q].y, m.x, acc[q][jj].y));
-        acc[q][jj + 1].x = fmaf(x[q].x, m.z, fmaf(-x[q].y, m.w, acc[q][jj + 1].x));
-        acc[q][jj + 1].y = fmaf(x[q].x, m.w, fmaf(x[q].y, m.z, acc[q][jj + 1].y));
-      }
-    }
-  } else {
+      for (int jj = 0; jj < NJ; ++jj) v[q][jj] = czero<C_t<R>>();
+  }
+  __device__ __forceinline__ void row(const C_t<R> (&x)[TG], const C_t<R>* __restrict__ mrow) {
 #pragma unroll
     for (int jj = 0; jj < NJ; ++jj) {
-      const double2 m = mrow[jj];
+      const C_t<R> m = mrow[jj];
 #pragma unroll
       for (int q = 0; q < TG; ++q) {
-        acc[q][jj].x = fma(x[q].x, m.x, fma(-x[q].y, m.y, acc[q][jj].x));
-        acc[q][jj].y = fma(x[q].x, m.y, fma(x[q].y, m.x, acc[q][jj].y));
+        v[q][jj].x = fma(x[q].x, m.x, fma(-x[q].y, m.y, v[q][jj].x));
+        v[q][jj].y = fma(x[q].x, m.y, fma(x[q].y, m.x, v[q][jj].y));
       }
     }
   }
-}
+  __device__ __forceinline__ C_t<R> get(int q, int jj) const { return v[q][jj]; }
+  static __device__ __forceinline__ void stage(C_t<R>* ms, int e, double2 m) { ms[e] = cmk<C_t<R>>(m.x, m.y); }
+};
+template <int NJ, int TG> struct RgAcc<float, NJ, TG> {
+  static_assert(NJ % 2 == 0, "column pairs");
+  float2 re[TG][NJ / 2], im[TG][NJ / 2];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int q = 0; q < TG; ++q)
+#pragma unroll
+      for (int j = 0; j < NJ / 2; ++j) re[q][j] = im[q][j] = make_float2(0.f, 0.f);
+  }
+  __device__ __forceinline__ void row(const float2 (&x)[TG], const float2* __restrict__ mrow) {
+#pragma unroll
+    for (int j = 0; j < NJ / 2; ++j) {
+      const float4 m = *reinterpret_cast<const float4*>(mrow + 2 * j);
+      const float2 mr = make_float2(m.x, m.y), mi = make_float2(m.z, m.w);
+#pragma unroll
+      for (int q = 0; q < TG; ++q) {
+        const float2 xr = make_float2(x[q].x, x[q].x), xi = make_float2(x[q].y, x[q].y),
+                     xn = make_float2(-x[q].y, -x[q].y);
+        re[q][j] = __ffma2_rn(xr, mr, __ffma2_rn(xn, mi, re[q][j]));
+        im[q][j] = __ffma2_rn(xr, mi, __ffma2_rn(xi, mr, im[q][j]));
+      }
+    }
+  }
+  __device__ __forceinline__ float2 get(int q, int jj) const {
+    return jj & 1 ? make_float2(re[q][jj / 2].y, im[q][jj / 2].y) : make_float2(re[q][jj / 2].x, im[q][jj / 2].x);
+  }
+  // element e = row * NJ + column of the M tile
+  static __device__ __forceinline__ void stage(float2* ms, int e, double2 m) {
+    float* f = reinterpret_cast<float*>(ms + (e & ~1)) + (e & 1);
+    f[0] = (float)m.x;
+    f[2] = (float)m.y;
+  }
+};
 
 // rows [lo, hi) of one term (lo a multiple of 4): X rows streamed RG at a
 // time, the next RG loaded before the current ones are used
 template <typename R, int LX, bool VIN, int NJ, int TG, int RG>
-__device__ __forceinline__ void rg_term(C_t<R> (&acc)[TG][NJ], const void* __restrict__ a,
+__device__ __forceinline__ void rg_term(RgAcc<R, NJ, TG>& acc, const void* __restrict__ a,
                                         const void* __restrict__ b, size_t sk, const int (&g)[TG], int ng, int nb,
                                         int lo, int hi, const C_t<R>* __restrict__ ms) {
   using C = C_t<R>;
@@ -113,7 +145,7 @@ __device__ __forceinline__ void rg_term(C_t<R> (&acc)[TG][NJ], const void* __res
       C x[TG];
 #pragma unroll
       for (int q = 0; q < TG; ++q) x[q] = cur[q][r];
-      rg_fma_row<R, NJ, TG>(acc, x, ms + (size_t)(k + r) * NJ);
+      acc.row(x, ms + (size_t)(k + r) * NJ);
     }
 #pragma unroll
     for (int q = 0; q < TG; ++q)
@@ -157,16 +189,18 @@ k_rotate_g(const void* __restrict__ X0a, const void* __restrict__ X0b, const dou
     double2 v = make_double2(0.0, 0.0);
     const bool in = term ? k < nb : (k >= lo0 && k < hi0);
     if (in && jj < nj) v = (term ? M1 : M0)[moff + (size_t)k * nb + j0 + jj];
-    ms[e] = cmk<C>(v.x, v.y);
+    RgAcc<R, NJ, TG>::stage(ms, e, v);
   }
   __syncthreads();
+  RgAcc<R, NJ, TG> sums;
+  sums.zero();
+  rg_term<R, LX0, VIN, NJ, TG, RG>(sums, X0a, X0b, sk, g, ng, nb, lo0 & ~3, hi0, ms);
+  if (X1) rg_term<R, RG_BAND, false, NJ, TG, RG>(sums, X1, nullptr, sk, g, ng, nb, 0, nb, ms + (size_t)nbp * NJ);
   C acc[TG][NJ];
 #pragma unroll
   for (int q = 0; q < TG; ++q)
 #pragma unroll
-    for (int jj = 0; jj < NJ; ++jj) acc[q][jj] = czero<C>();
-  rg_term<R, LX0, VIN, NJ, TG, RG>(acc, X0a, X0b, sk, g, ng, nb, lo0 & ~3, hi0, ms);
-  if (X1) rg_term<R, RG_BAND, false, NJ, TG, RG>(acc, X1, nullptr, sk, g, ng, nb, 0, nb, ms + (size_t)nbp * NJ);
+    for (int jj = 0; jj < NJ; ++jj) acc[q][jj] = sums.get(q, jj);
 
   if constexpr (OUT == RG_BANDMAJOR) {
 #pragma unroll
@@ -338,7 +372,8 @@ static int rg_go(const void* X0a, const void* X0b, const double2* M0, const void
 // Tile shapes: the band count rounded up to 8, at most 32 (FP32) or 16
 // (FP64) columns per tile, one G vector per thread (two G vectors per thread
 // with 8- or 12-column tiles measured within 1 % at 24 bands and slower at
-// 160 bands, where more tiles re-read X; 16-column tiles at three CTAs per
+// 160 bands, where more tiles re-read X; with 24 or 32 columns 296 vs 220 us
+// (Si8 adjoint and Adam) and 4.70 vs 4.47 ms (Si64); 16-column tiles at three CTAs per
 // SM slower at 24 bands).
 template <typename R, int LX0, int OUT>
 static int rg_pick(const void* X0a, const void* X0b, const double2* M0, const void* X1, const double2* M1,
@@ -350,7 +385,17 @@ static int rg_pick(const void* X0a, const void* X0b, const double2* M0, const vo
   // adjoint keeps one tile
   if (sizeof(R) == 4 && OUT == RG_BANDMAJOR && nb <= 32) return rg_go<R, LX0, OUT, 8, 1, 4>(RG_ARGS);
   if (nb <= 8) return rg_go<R, LX0, OUT, 8, 1, 2>(RG_ARGS);
-  if (sizeof(R) == 8 || nb <= 16) return rg_go<R, LX0, OUT, 16, 1, 2>(RG_ARGS);
+  if constexpr (sizeof(R) == 8) {
+    // FP64 is bound by its arithmetic: tiles of at most 16 columns, as even and as
+    // narrow as the bands allow (243 bands in blocks of 9: 16 columns computed 44 %
+    // for nothing)
+    const int tiles = (nb + 15) / 16, w = (nb + tiles - 1) / tiles;
+    if (w <= 10) return rg_go<R, LX0, OUT, 10, 1, 2>(RG_ARGS);
+    if (w <= 12) return rg_go<R, LX0, OUT, 12, 1, 2>(RG_ARGS);
+    if (w <= 14) return rg_go<R, LX0, OUT, 14, 1, 2>(RG_ARGS);
+    return rg_go<R, LX0, OUT, 16, 1, 2>(RG_ARGS);
+  }
+  if (nb <= 16) return rg_go<R, LX0, OUT, 16, 1, 2>(RG_ARGS);
   if (nb <= 24) return rg_go<R, LX0, OUT, 24, 1, 2>(RG_ARGS);
   return rg_go<R, LX0, OUT, 32, 1, 2>(RG_ARGS);
 #undef RG_ARGS
