@@ -181,12 +181,16 @@ size_t gram_w_smem(int NBP, bool same = false) {
 }
 
 // SAME: Y is X (W^H W): the chunk is staged once.
-template <typename R, int LX, int LY, int NBP, bool SAME = false>
+// UP: only the blocks that reach the diagonal or above are formed and the rest is
+// their conjugate transpose: W^H W is Hermitian, and of C^H g_C only the upper
+// triangle and the diagonal are read (a third fewer products at 24 bands).  TI: row
+// blocks of four (FP64, bound by its arithmetic, takes no more than the bands need).
+template <typename R, int LX, int LY, int NBP, bool SAME, bool UP, int TI = NBP / 4>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1)
 k_gram_w(const void* __restrict__ X0, const void* __restrict__ X1, const void* __restrict__ Y0,
          const void* __restrict__ Y1, double2* __restrict__ part, int ng, int nb, int split_len) {
   using C = C_t<R>;
-  constexpr int CG = kGwCG, LD = NBP + 1, TI = NBP / 4, TJ = NBP / 8;
+  constexpr int CG = kGwCG, LD = NBP + 1, TJ = NBP / 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* xs = reinterpret_cast<C*>(smem_raw);   // [2][CG][LD]
   C* ys = SAME ? xs : xs + 2 * CG * LD;     // [2][CG][LD]
@@ -297,6 +301,7 @@ k_gram_w(const void* __restrict__ X0, const void* __restrict__ X1, const void* _
       for (int a = 0; a < TI; ++a)
 #pragma unroll
         for (int b = 0; b < TJ; ++b) {   // conj(x) * y
+          if (UP && 4 * a > 8 * b + 7) continue;
           acc[a][b].x = fma(x[a].x, y[b].x, fma(x[a].y, y[b].y, acc[a][b].x));
           acc[a][b].y = fma(x[a].x, y[b].y, fma(-x[a].y, y[b].x, acc[a][b].y));
         }
@@ -317,12 +322,12 @@ k_gram_w(const void* __restrict__ X0, const void* __restrict__ X1, const void* _
     const int i = e / nb, j = e - i * nb;
     C u[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) u[q] = red[((size_t)q * NBP + i) * NBP + j];
+    for (int q = 0; q < 8; ++q) u[q] = red[((size_t)q * NBP + (UP ? min(i, j) : i)) * NBP + (UP ? max(i, j) : j)];
 #pragma unroll
     for (int h = 4; h > 0; h >>= 1)
 #pragma unroll
       for (int q = 0; q < h; ++q) { u[q].x += u[q + h].x; u[q].y += u[q + h].y; }
-    part[(sk * nsplit + split) * nn + e] = make_double2((double)u[0].x, (double)u[0].y);
+    part[(sk * nsplit + split) * nn + e] = make_double2((double)u[0].x, UP && i > j ? -(double)u[0].y : (double)u[0].y);
   }
 }
 
@@ -1073,16 +1078,22 @@ int launch_gram(int lx, const void* X0, const void* X1, int ly, const void* Y0, 
     };
     auto pick = [&](auto lxc, auto lyc) -> int {
       constexpr int A = decltype(lxc)::value, B = decltype(lyc)::value;
-      if (same) {
-        if (nb <= 8) return go(k_gram_w<R, A, B, 8, true>, 8);
-        if (nb <= 16) return go(k_gram_w<R, A, B, 16, true>, 16);
-        if (nb <= 24) return go(k_gram_w<R, A, B, 24, true>, 24);
-        return go(k_gram_w<R, A, B, 32, true>, 32);
-      }
-      if (nb <= 8) return go(k_gram_w<R, A, B, 8>, 8);
-      if (nb <= 16) return go(k_gram_w<R, A, B, 16>, 16);
-      if (nb <= 24) return go(k_gram_w<R, A, B, 24>, 24);
-      return go(k_gram_w<R, A, B, 32>, 32);
+      auto size = [&](auto samec, auto upc) -> int {
+        constexpr bool S = decltype(samec)::value, U = decltype(upc)::value;
+        if constexpr (sizeof(R) == 8) {
+          if (nb <= 4) return go(k_gram_w<R, A, B, 8, S, U, 1>, 8);
+          if (nb > 8 && nb <= 12) return go(k_gram_w<R, A, B, 16, S, U, 3>, 16);
+          if (nb > 16 && nb <= 20) return go(k_gram_w<R, A, B, 24, S, U, 5>, 24);
+          if (nb > 24 && nb <= 28) return go(k_gram_w<R, A, B, 32, S, U, 7>, 32);
+        }
+        if (nb <= 8) return go(k_gram_w<R, A, B, 8, S, U>, 8);
+        if (nb <= 16) return go(k_gram_w<R, A, B, 16, S, U>, 16);
+        if (nb <= 24) return go(k_gram_w<R, A, B, 24, S, U>, 24);
+        return go(k_gram_w<R, A, B, 32, S, U>, 32);
+      };
+      if (same) return size(std::true_type{}, std::true_type{});
+      if (!full) return size(std::false_type{}, std::true_type{});
+      return size(std::false_type{}, std::false_type{});
     };
     int rc;
     if (lx == LAYOUT_SPLIT && ly == LAYOUT_SPLIT)
