@@ -279,6 +279,10 @@ int jrg_lda_polarized(int precision, int64_t n, int xc, int kohn_sham, const voi
 int jrg_fft3d_workspace_size(int precision, const int grid[3], int batch, size_t* bytes);
 int jrg_fft3d(int precision, const int grid[3], int batch, int direction, const void* in,
               void* out, void* workspace, cudaStream_t stream);
+/* jrg_fft3d with any factor in place of 1 or 1/(nx ny nz), applied in the last
+ * pass (pw.wave_grid's 1/sqrt(vol), jrystal/_src/pw.py:140-211). */
+int jrg_fft3d_scaled(int precision, const int grid[3], int batch, int direction, double scale, const void* in,
+                     void* out, void* workspace, cudaStream_t stream);
 
 /* jrg_fft3d without a workspace, for callers that cannot allocate device
  * memory (a runtime that owns the device memory, a fixed memory budget, or a

@@ -98,6 +98,8 @@ _SIGS = {
                                 ct.POINTER(ct.c_size_t)], ct.c_int),
   "jrg_fft3d": ([ct.c_int, ct.POINTER(ct.c_int), ct.c_int, ct.c_int, _vp, _vp, _vp,
                  _vp], ct.c_int),
+  "jrg_fft3d_scaled": ([ct.c_int, ct.POINTER(ct.c_int), ct.c_int, ct.c_int, ct.c_double, _vp, _vp, _vp,
+                        _vp], ct.c_int),
   "jrg_fft3d_noalloc": ([ct.c_int, ct.POINTER(ct.c_int), ct.c_int, ct.c_int, _vp, _vp, _vp],
                         ct.c_int),
   "jrg_lda": ([ct.c_int, ct.c_int64, ct.c_int, ct.c_int, _vp, _vp, _vp], ct.c_int),

@@ -91,6 +91,24 @@ class _Fft3(torch.autograd.Function):
     return _fft3d(g, inverse=True) * ctx.n, None   # y = F x  ->  x_bar = conj(F) y_bar
 
 
+class _WaveFft(torch.autograd.Function):
+  """scale * sum_G c_G exp(iG.r) in one transform (no pass for the factor)."""
+
+  @staticmethod
+  def forward(ctx, x, scale):
+    ctx.scale = scale
+    return _fft3d(x.contiguous(), inverse=True, scale=scale)
+
+  @staticmethod
+  def backward(ctx, g):
+    return _fft3d(g.contiguous(), inverse=False, scale=ctx.scale), None
+
+
+def wave_fft(x: torch.Tensor, scale: float) -> torch.Tensor:
+  """Unnormalised inverse FFT over the last three axes times ``scale``."""
+  return _WaveFft.apply(_complex(x), float(scale))
+
+
 def _complex(x: torch.Tensor) -> torch.Tensor:
   if torch.is_complex(x):
     return x

@@ -1426,8 +1426,8 @@ int jrg_fft3d_workspace_size(int prec, const int grid[3], int batch, size_t* byt
   return JRG_OK;
 }
 
-int jrg_fft3d(int prec, const int grid[3], int batch, int direction, const void* in, void* out,
-              void* ws, cudaStream_t st) {
+int jrg_fft3d_scaled(int prec, const int grid[3], int batch, int direction, double scale, const void* in,
+                     void* out, void* ws, cudaStream_t st) {
   if (!grid || !in || !out || !ws || batch < 1 || (direction != 1 && direction != -1) ||
       (prec != 32 && prec != 64))
     return fail(JRG_ERR_INVALID, "jrg_fft3d: bad argument");
@@ -1454,12 +1454,17 @@ int jrg_fft3d(int prec, const int grid[3], int batch, int direction, const void*
     off += grid[a];
   }
   if (rc) return rc;
-  const double scale = direction > 0 ? 1.0 / ((double)grid[0] * grid[1] * grid[2]) : 1.0;
   if (prec == 64)
     return launch_fft3d_dense<double>(ax, (const double2*)tw, batch, direction, false, in,
                                       (double2*)scratch, (double2*)out, scale, st);
   return launch_fft3d_dense<float>(ax, (const float2*)tw, batch, direction, false, in,
                                    (float2*)scratch, (float2*)out, scale, st);
+}
+int jrg_fft3d(int prec, const int grid[3], int batch, int direction, const void* in, void* out,
+              void* ws, cudaStream_t st) {
+  if (!grid) return fail(JRG_ERR_INVALID, "jrg_fft3d: bad argument");
+  const double scale = direction > 0 ? 1.0 / ((double)grid[0] * grid[1] * grid[2]) : 1.0;
+  return jrg_fft3d_scaled(prec, grid, batch, direction, scale, in, out, ws, st);
 }
 
 int jrg_precond_scale(const jrg_plan* P, const float* w32, const void* wb, float t_frac, float smax,

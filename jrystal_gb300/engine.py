@@ -383,8 +383,9 @@ class PlaneWavePlan:
       pass
 
 
-def fft3d(x: torch.Tensor, inverse: bool = False) -> torch.Tensor:
-  """Complex FFT over the last three axes (jnp.fft.fftn / ifftn semantics)."""
+def fft3d(x: torch.Tensor, inverse: bool = False, scale: Optional[float] = None) -> torch.Tensor:
+  """Complex FFT over the last three axes (jnp.fft.fftn / ifftn semantics; with
+  ``scale``, the unnormalised sum times it)."""
   lib = _lib.load()
   if not x.is_cuda:
     raise RuntimeError("fft3d needs a CUDA tensor (no CPU fallback)")
@@ -398,8 +399,12 @@ def fft3d(x: torch.Tensor, inverse: bool = False) -> torch.Tensor:
   _lib.check(lib.jrg_fft3d_workspace_size(prec, grid, batch, ct.byref(nbytes)), "jrg_fft3d_workspace_size")
   ws = torch.empty(int(nbytes.value), dtype=torch.uint8, device=x.device)
   out = torch.empty_like(x)
-  _lib.check(lib.jrg_fft3d(prec, grid, batch, 1 if inverse else -1, _ptr(x), _ptr(out), _ptr(ws),
-                           _stream()), "jrg_fft3d")
+  if scale is None:
+    st = lib.jrg_fft3d(prec, grid, batch, 1 if inverse else -1, _ptr(x), _ptr(out), _ptr(ws), _stream())
+  else:
+    st = lib.jrg_fft3d_scaled(prec, grid, batch, 1 if inverse else -1, float(scale), _ptr(x), _ptr(out),
+                              _ptr(ws), _stream())
+  _lib.check(st, "jrg_fft3d")
   return out
 
 

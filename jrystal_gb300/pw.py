@@ -8,7 +8,7 @@ import numpy as np
 import torch
 
 from . import plans
-from ._ops import as_tensor, fftn, get_precision, ifftn, precision_of, real_dtype, to_numpy
+from ._ops import as_tensor, fftn, get_precision, precision_of, real_dtype, to_numpy, wave_fft
 from .grid import g_vectors
 from .utils import absolute_square, expand_coefficient, volume
 
@@ -88,9 +88,7 @@ def coeff(pw_param, freq_mask, sharding=None) -> torch.Tensor:
 
 def wave_grid(coeff, vol) -> torch.Tensor:
   """IFFT_3(c) * N / sqrt(vol) (pw.py:140-211)."""
-  c = as_tensor(coeff)
-  n = float(np.prod(c.shape[-3:]))
-  return ifftn(c) * (n / np.sqrt(float(vol)))
+  return wave_fft(as_tensor(coeff), 1.0 / np.sqrt(float(vol)))
 
 
 def density_grid(coeff, vol, occupation=None) -> torch.Tensor:

@@ -107,3 +107,26 @@ def test_band_trace_with_zero_weights():
       plan.lib.jrg_fast_paths(prev)
   for x, y in zip(*out):
     assert np.linalg.norm(x - y) <= 1.4e-14 * np.linalg.norm(y)
+
+
+@pytest.mark.parametrize("prec", [32, 64])
+@pytest.mark.parametrize("shape", [(1, 2, 3, 24, 24, 24), (5, 20, 27, 16), (16, 16, 16)])
+def test_wave_grid_and_its_adjoint(shape, prec):
+  """Factor applied inside the transform, value and vector-Jacobian product against
+  numpy (a transform's rounding, 24 log2(N) eps at most)."""
+  import torch
+  from jrystal_gb300 import pw
+  rng = np.random.default_rng(4)
+  z = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+  g = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+  dt = torch.complex64 if prec == 32 else torch.complex128
+  c = torch.tensor(z, dtype=dt, device="cuda", requires_grad=True)
+  w = pw.wave_grid(c, 37.5)
+  w.backward(torch.tensor(g, dtype=dt, device="cuda"))
+  ax = (-3, -2, -1)
+  n = np.prod(shape[-3:])
+  tol = 24 * np.log2(n) * (1.2e-7 if prec == 32 else 2.2e-16)
+  want = np.fft.ifftn(z, axes=ax) * n / np.sqrt(37.5)
+  adj = np.fft.fftn(g, axes=ax) / np.sqrt(37.5)
+  for a, b in ((w.detach(), want), (c.grad, adj)):
+    assert np.linalg.norm(a.cpu().numpy() - b) <= tol * np.linalg.norm(b)
