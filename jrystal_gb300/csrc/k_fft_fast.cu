@@ -646,6 +646,82 @@ __global__ void __launch_bounds__(threads_for<N>()) k_line_dense(const C_t<R>* _
   for (int j = 0; j < N1; ++j) out[base + (size_t)(N2 * j + j2) * (N * N)] = cscale(v[j], sc);
 }
 
+static int optin_smem() {
+  int dev = 0, v = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  return v;
+}
+
+// 1: ready to launch, 0: does not fit (use the generic kernels), <0: -status
+template <typename K> static int prep(K kernel, size_t bytes) {
+  if ((long long)bytes > optin_smem()) return 0;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             (int)cudaSharedmemCarveoutMaxShared);
+  if (e != cudaSuccess) return -cuda_fail(e, "cudaFuncSetAttribute(fast slab kernel)");
+  return 1;
+}
+
+#define FAST_LAUNCHED(what)                                  \
+  do {                                                       \
+    ::jrg::count_launch();                                   \
+    cudaError_t e_ = cudaGetLastError();                     \
+    if (e_ != cudaSuccess) return -::jrg::cuda_fail(e_, what); \
+    return 1;                                                \
+  } while (0)
+
+// Transforms along one axis of a whole grid, kAxisLines lines a CTA (axis 0, 1, 2: x,
+// y, z), in place or not, times scale.  For single FP64 grids: they are bound by
+// FP64 arithmetic (two operations a cycle and SM), and one CTA per plane leaves
+// most SMs without work (48^3: plane pass 30 us on 48 SMs, two axis passes 2 x 5).
+constexpr int kAxisLines = 16;
+template <typename R, int N, int DIR, bool REAL_IN>
+__global__ void __launch_bounds__(kAxisLines * Split<N>::N2) k_axis_lines(const void* in_v, C_t<R>* out,
+                                                                          const C_t<R>* __restrict__ tw_g, int axis,
+                                                                          double scale) {
+  using C = C_t<R>;
+  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2, L = kAxisLines;
+  __shared__ C tw[N];
+  __shared__ C ex[N * L];
+  const int tid = threadIdx.x, l = blockIdx.x * L + tid % L, j2 = tid / L;
+  const bool act = l < N * N;
+  // line l: (y, z), (x, z) or (x, y) of the axis
+  const int es = axis == 0 ? N * N : (axis == 1 ? N : 1);
+  const int base = axis == 0 ? l : (axis == 1 ? l / N * (N * N) + l % N : l * N);
+  for (int i = tid; i < N; i += blockDim.x) tw[i] = tw_g[i];
+  C v[N1];
+#pragma unroll
+  for (int j1 = 0; j1 < N1; ++j1) {
+    v[j1] = czero<C>();
+    if (act) {
+      const int i = base + (N2 * j1 + j2) * es;
+      if constexpr (REAL_IN) v[j1].x = reinterpret_cast<const R*>(in_v)[i];
+      else v[j1] = reinterpret_cast<const C*>(in_v)[i];
+    }
+  }
+  __syncthreads();
+  reg::line_step_a<N, DIR>(v, tw, j2, ex, L, tid % L);
+  __syncthreads();
+  reg::line_step_b<N, DIR>(v, j2, ex, L, tid % L);
+  const R sc = (R)scale;
+  if (act) {
+#pragma unroll
+    for (int j = 0; j < N1; ++j) out[base + (N2 * j + j2) * es] = cscale(v[j], sc);
+  }
+}
+template <typename R, int N, int DIR, bool REAL_IN>
+static int axis_pass(const void* in, C_t<R>* out, const C_t<R>* tw, int axis, double scale, cudaStream_t st) {
+  k_axis_lines<R, N, DIR, REAL_IN><<<(N * N + kAxisLines - 1) / kAxisLines, kAxisLines * Split<N>::N2, 0, st>>>(
+      in, out, tw, axis, scale);
+  FAST_LAUNCHED("fast::k_axis_lines");
+}
+// single FP64 grids from 48^3 (density and potentials of a 48^3 state 593 -> 567 us);
+// at 32^3 a plane pass takes 10 us and the launch more costs what it gives (PBE's
+// nine transforms: 1694 us a step by planes, 1717 by axes)
+template <typename R, int N> static bool by_axes(int batch) { return sizeof(R) == 8 && batch == 1 && N >= 48; }
+
 // x forward, Hartree term, x inverse of one (y, half of z) of a density
 // transformed in y and z, in place (the Hartree term of k_recip_terms between two
 // dense line passes): V_H(G) = inv_n s ginv rho(G), E_H partials of the CTA in
@@ -719,32 +795,6 @@ template <typename R, int N> size_t line_smem() {
 template <typename R, int N> size_t line_pf_smem(int nact) {
   return line_pf_offset<R, N>() + 2 * sizeof(C_t<R>) * (size_t)nact * N;
 }
-
-static int optin_smem() {
-  int dev = 0, v = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  return v;
-}
-
-// 1: ready to launch, 0: does not fit (use the generic kernels), <0: -status
-template <typename K> static int prep(K kernel, size_t bytes) {
-  if ((long long)bytes > optin_smem()) return 0;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
-  if (e != cudaSuccess) return -cuda_fail(e, "cudaFuncSetAttribute(fast slab kernel)");
-  return 1;
-}
-
-#define FAST_LAUNCHED(what)                                  \
-  do {                                                       \
-    ::jrg::count_launch();                                   \
-    cudaError_t e_ = cudaGetLastError();                     \
-    if (e_ != cudaSuccess) return -::jrg::cuda_fail(e_, what); \
-    return 1;                                                \
-  } while (0)
 
 static bool g_line_prefetch = true;   // cp.async row prefetch in the adjoint line kernel
 
@@ -936,6 +986,15 @@ static int dense_run(const C_t<R>* tw, int batch, bool real_in, const void* in, 
   const size_t smp = sizeof(C) * (size_t)(N + N * (N + 1) + N * N);
   const size_t sml = sizeof(C) * (size_t)(N + N * N);
   int rc;
+  if constexpr (sizeof(R) == 8 && N >= 48 && N <= 64) {
+    if (by_axes<R, N>(batch)) {
+      rc = real_in ? axis_pass<R, N, DIR, true>(in, scratch, tw, 2, 1.0, st)
+                   : axis_pass<R, N, DIR, false>(in, scratch, tw, 2, 1.0, st);
+      if (rc > 0) rc = axis_pass<R, N, DIR, false>(scratch, scratch, tw, 1, 1.0, st);
+      if (rc > 0) rc = axis_pass<R, N, DIR, false>(scratch, out, tw, 0, scale, st);
+      return rc;
+    }
+  }
   if (real_in) {
     if ((rc = prep(k_plane_dense<R, N, DIR, true>, smp)) <= 0) return rc;
     k_plane_dense<R, N, DIR, true><<<dim3(N, batch), T, smp, st>>>(in, scratch, tw);
@@ -992,6 +1051,18 @@ static int hartree_run(const C_t<R>* tw, const void* rho, C_t<R>* mid, C_t<R>* r
   const size_t smp = sizeof(C) * (size_t)(N + N * (N + 1) + N * N), sml = sizeof(C) * (size_t)N * L;
   if (N * (N / L) > nslots) return 0;
   int rc;
+  if constexpr (sizeof(R) == 8 && N >= 48 && N <= 64) {
+    if (by_axes<R, N>(1)) {
+      if ((rc = prep(k_line_hartree<R, N>, sml)) <= 0) return rc;
+      if ((rc = axis_pass<R, N, -1, true>(rho, mid, tw, 2, 1.0, st)) <= 0) return rc;
+      if ((rc = axis_pass<R, N, -1, false>(mid, mid, tw, 1, 1.0, st)) <= 0) return rc;
+      k_line_hartree<R, N><<<dim3(N, N / L), hartree_threads<N>(), sml, st>>>(mid, tw, ginv, slot_h, nslots, pref,
+                                                                             inv_n, cf);
+      ::jrg::count_launch();
+      if ((rc = axis_pass<R, N, +1, false>(mid, mid, tw, 1, 1.0, st)) <= 0) return rc;
+      return axis_pass<R, N, +1, false>(mid, rhog, tw, 2, 1.0, st);
+    }
+  }
   if ((rc = prep(k_plane_dense<R, N, -1, true>, smp)) <= 0) return rc;
   if ((rc = prep(k_plane_dense<R, N, +1, false>, smp)) <= 0) return rc;
   if ((rc = prep(k_line_hartree<R, N>, sml)) <= 0) return rc;
