@@ -22,10 +22,10 @@ template <typename R> int launch_hartree(const jrg_plan*, const void*, C_t<R>*, 
 template <typename R> int launch_adam_pair(const AdamArgs&, size_t, const void*, const void*, long long, cudaStream_t);
 template <typename R> int launch_pack_params(const void*, const void*, void*, int, int, int, bool, cudaStream_t);
 template <typename R> int launch_unpack(const void*, void*, void*, void*, int, int, int, double, cudaStream_t);
-template <typename R> int launch_gram(int, const void*, const void*, int, const void*, const void*, double2*, double2*, int, int, int, int, cudaStream_t, int* = nullptr, bool = false);
-int launch_cholesky_inv(const double2*, double2*, double2*, int, int, int*, double*, cudaStream_t, double, bool);
+template <typename R> int launch_gram(int, const void*, const void*, int, const void*, const void*, double2*, double2*, int, int, int, int, cudaStream_t, int* = nullptr, bool = false, int* = nullptr);
+int launch_cholesky_inv(const double2*, double2*, double2*, int, int, int*, double*, cudaStream_t, double, bool, int = 0);
 int launch_adjoint_small(const double2*, const double2*, double2*, double2*, int, int, cudaStream_t,
-                         const double* = nullptr, double* = nullptr);
+                         const double* = nullptr, double* = nullptr, int = 0);
 template <typename R> int launch_rotate(int, int, const void*, const void*, const double2*, const void*, const double2*, void*, void*, int, int, int, double, void*, cudaStream_t, int = 0);
 constexpr int kTriUpper = 1, kTriLower = 2;   // zero pattern of a rotation's first matrix: R^-1, R^-H
 constexpr int kSplit = 0, kBand = 1;           // tall-operand layouts (k_orth.cu)
@@ -646,19 +646,19 @@ static int orthonormalise(const jrg_plan* P, const void* w_re, const void* w_im,
                           int* kin_blocks = nullptr) {
   const Workspace& w = P->ws;
   const int nsk = P->ns * P->nk;
-  int rc;
+  int rc, fold = 0;
   {
     PHASE(PH_GRAM);
     if ((rc = launch_gram<R>(kSplit, w_re, w_im, kSplit, w_re, w_im, (double2*)wsp(ws, w.gram_part),
                              (double2*)wsp(ws, w.gram), nsk, P->ng, P->nb, w.gram_splits, st,
-                             (int*)wsp(ws, w.flags))))
+                             (int*)wsp(ws, w.flags), false, &fold)))
       return rc;
   }
   {
     PHASE(PH_CHOL);
-    if ((rc = launch_cholesky_inv((double2*)wsp(ws, w.gram), (double2*)wsp(ws, w.rmat),
+    if ((rc = launch_cholesky_inv((double2*)wsp(ws, fold ? w.gram_part : w.gram), (double2*)wsp(ws, w.rmat),
                                   (double2*)wsp(ws, w.rinv), nsk, P->nb, (int*)wsp(ws, w.flags),
-                                  (double*)wsp(ws, w.dinv), st, min_pivot(P), P->prec == 32)))
+                                  (double*)wsp(ws, w.dinv), st, min_pivot(P), P->prec == 32, fold)))
       return rc;
   }
   PHASE(PH_ROTATE);
@@ -1066,14 +1066,16 @@ static int phase_forward_range(const jrg_plan* P, const void* w_re, const void* 
   const R* wi = reinterpret_cast<const R*>(w_im) + po;
   int* flags = (int*)wsp(ws, w.flags);
   int rc;
-  if ((rc = launch_gram<R>(kSplit, wr, wi, kSplit, wr, wi,
-                           (double2*)wsp(ws, w.gram_part) + (size_t)k0 * w.gram_splits * nb2,
-                           (double2*)wsp(ws, w.gram) + k0 * nb2, n, P->ng, P->nb, w.gram_splits, st,
-                           flags)))
+  int fold = 0;
+  double2* part = (double2*)wsp(ws, w.gram_part) + (size_t)k0 * w.gram_splits * nb2;
+  double2* gram = (double2*)wsp(ws, w.gram) + k0 * nb2;
+  if ((rc = launch_gram<R>(kSplit, wr, wi, kSplit, wr, wi, part, gram, n, P->ng, P->nb, w.gram_splits, st, flags,
+                           false, &fold)))
     return rc;
-  if ((rc = launch_cholesky_inv((double2*)wsp(ws, w.gram) + k0 * nb2, (double2*)wsp(ws, w.rmat) + k0 * nb2,
+  if ((rc = launch_cholesky_inv(fold ? part : gram, (double2*)wsp(ws, w.rmat) + k0 * nb2,
                                 (double2*)wsp(ws, w.rinv) + k0 * nb2, n, P->nb, flags,
-                                (double*)wsp(ws, w.dinv) + (size_t)k0 * P->nb, st, min_pivot(P), P->prec == 32)))
+                                (double*)wsp(ws, w.dinv) + (size_t)k0 * P->nb, st, min_pivot(P), P->prec == 32,
+                                fold)))
     return rc;
   const int kb = launch_rotate_kinetic<R>(wr, wi, (double2*)wsp(ws, w.rinv) + k0 * nb2,
                                           (C*)wsp(ws, w.c) + co, n, P->ng, P->nb, P->d.tk, P->nk,
@@ -1110,15 +1112,16 @@ static int phase_adjoint_range(const jrg_plan* P, const double* occ, void* g_re,
   if ((rc = apply_v_blocks<R>(P, t, t, wsp(ws, w.vr), occ, k0, n, st))) return rc;
   if ((rc = launch_plane_fwd_sphere<R>(P, t, c, gc, occ, k0 * P->nb, n * P->nb, 1.0 / N, st))) return rc;
   if ((rc = nl_adjoint<R>(P, ws, k0, n, st))) return rc;
-  if ((rc = launch_gram<R>(kBand, c, nullptr, kBand, gc, nullptr,
-                           (double2*)wsp(ws, w.adj_part) + (size_t)k0 * w.gram_splits * nb2,
-                           (double2*)wsp(ws, w.adj) + k0 * nb2, n, P->ng, P->nb, w.gram_splits, st,
-                           (int*)wsp(ws, w.flags))))
+  int fold = 0;
+  double2* part = (double2*)wsp(ws, w.adj_part) + (size_t)k0 * w.gram_splits * nb2;
+  double2* adj = (double2*)wsp(ws, w.adj) + k0 * nb2;
+  if ((rc = launch_gram<R>(kBand, c, nullptr, kBand, gc, nullptr, part, adj, n, P->ng, P->nb, w.gram_splits, st,
+                           (int*)wsp(ws, w.flags), false, P->nb <= 16 ? &fold : nullptr)))
     return rc;
   double2* rh = (double2*)wsp(ws, w.kmat);
   double2* negm2 = rh + (size_t)nsk * nb2;
-  if ((rc = launch_adjoint_small((double2*)wsp(ws, w.adj) + k0 * nb2, (double2*)wsp(ws, w.rinv) + k0 * nb2,
-                                 rh + k0 * nb2, negm2 + k0 * nb2, n, P->nb, st)))
+  if ((rc = launch_adjoint_small(fold ? part : adj, (double2*)wsp(ws, w.rinv) + k0 * nb2, rh + k0 * nb2,
+                                 negm2 + k0 * nb2, n, P->nb, st, nullptr, nullptr, fold)))
     return rc;
   const size_t cnt = (size_t)n * P->ng * P->nb;
   R* gr = adam ? (adam->grad[0] ? reinterpret_cast<R*>(adam->grad[0]) + po : reinterpret_cast<R*>(t))

@@ -74,10 +74,6 @@ __device__ __forceinline__ dc ld(const float4* p) {
   return {{v.x, v.y}, {v.z, v.w}};
 }
 __device__ __forceinline__ void st(float4* p, dc a) { *p = make_float4(a.re.hi, a.re.lo, a.im.hi, a.im.lo); }
-__device__ __forceinline__ dc cmul(dc a, dc b) {
-  return {add(mul(a.re, b.re), neg(mul(a.im, b.im))), add(mul(a.re, b.im), mul(a.im, b.re))};
-}
-__device__ __forceinline__ dc csub(dc a, dc b) { return {add(a.re, neg(b.re)), add(a.im, neg(b.im))}; }
 __device__ __forceinline__ dc cscale(dc a, df s) { return {mul(a.re, s), mul(a.im, s)}; }
 __device__ __forceinline__ dc conj(dc a) { return {a.re, neg(a.im)}; }
 
@@ -127,7 +123,7 @@ __device__ __forceinline__ double rsqrt_nr(double d) {
 template <int NT>
 __global__ void __launch_bounds__(NT, 1)
 k_cholesky_inv_df(const double2* __restrict__ S, double2* __restrict__ Ri, int nb, int* __restrict__ flags,
-                  double min_pivot) {
+                  double min_pivot, int nsplit) {
   using namespace dfa;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // FP64 work stays off the per-element paths (1/64 of the FP32 rate): the
@@ -140,10 +136,15 @@ k_cholesky_inv_df(const double2* __restrict__ S, double2* __restrict__ Ri, int n
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = NT / 32;
   const size_t off = (size_t)blockIdx.x * nb * nb;
   auto idx = [nb](int i, int j) { return i * (2 * nb - i - 1) / 2 + j; };
-  // upper triangle of the Hermitian part of S
+  // upper triangle of the Hermitian part of S, the sum of nsplit parts
+  const double2* s0 = S + off * nsplit;
   for (int i = warp; i < nb; i += nwarp)
     for (int j = i + lane; j < nb; j += 32) {
-      const double2 a = S[off + (size_t)i * nb + j], b = S[off + (size_t)j * nb + i];
+      double2 a = s0[i * nb + j], b = s0[j * nb + i];
+      for (int p = 1; p < nsplit; ++p) {
+        const double2 u = s0[p * nb * nb + i * nb + j], v = s0[p * nb * nb + j * nb + i];
+        a.x += u.x; a.y += u.y; b.x += v.x; b.y += v.y;
+      }
       const double re = 0.5 * (a.x + b.x), im = i == j ? 0.0 : 0.5 * (a.y - b.y);
       st(U + idx(i, j), dc{from_d(re), from_d(im)});
       if (i == j) { sdiag[i] = a.x; thr[i] = (float)(min_pivot * a.x); }
@@ -232,7 +233,7 @@ k_cholesky_inv_df(const double2* __restrict__ S, double2* __restrict__ Ri, int n
 // 1: launched; 0: the triangle does not fit in shared memory (use the FP64
 // kernel); < 0: -status
 int launch_cholesky_inv_df(const double2* S, double2* Ri, int nsk, int nb, int* flags, double min_pivot,
-                           cudaStream_t st) {
+                           cudaStream_t st, int nsplit) {
   const size_t sm = chol_df_smem(nb);
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
@@ -242,7 +243,7 @@ int launch_cholesky_inv_df(const double2* S, double2* Ri, int nsk, int nb, int* 
   auto go = [&](auto kern, int nt) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    kern<<<nsk, nt, sm, st>>>(S, Ri, nb, flags, min_pivot);
+    kern<<<nsk, nt, sm, st>>>(S, Ri, nb, flags, min_pivot, nsplit);
     return cudaSuccess;
   };
   cudaError_t e = nb <= 64 ? go(k_cholesky_inv_df<256>, 256) : go(k_cholesky_inv_df<1024>, 1024);

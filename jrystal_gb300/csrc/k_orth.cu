@@ -544,10 +544,23 @@ __global__ void __launch_bounds__(kAdjSmallThreads) k_adjoint_small(const double
                                                        double2* __restrict__ Rh,
                                                        double2* __restrict__ negM2, int nb,
                                                        const double* __restrict__ f,
-                                                       double* __restrict__ eps, bool with_m2) {
+                                                       double* __restrict__ eps, bool with_m2, int fold) {
   const int sk = blockIdx.x;
   const size_t off = (size_t)sk * nb * nb;
+  // fold > 0: A holds the splits of the Gram product (nb <= 16), summed here
+  __shared__ double2 sa[16 * 16];
   const double2* a = A + off;
+  if (fold > 0) {
+    const int nn = nb * nb;
+    const double2* p = A + off * fold;
+    for (int e = threadIdx.x; e < nn; e += blockDim.x) {
+      double2 v = p[e];
+      for (int q = 1; q < fold; ++q) { v.x += p[q * nn + e].x; v.y += p[q * nn + e].y; }
+      sa[e] = v;
+    }
+    __syncthreads();
+    a = sa;
+  }
   const double2* ri = Ri + off;
   const double* fb = f ? f + (size_t)sk * nb : nullptr;
   auto fw = [&](int j) { return fb ? fb[j] : 1.0; };
@@ -1034,6 +1047,11 @@ static bool g_gram_rb = true;       // register-blocked Gram for B <= 32 (else 3
 static bool g_rotate_rb = true;     // register-blocked rotation for B <= 32
 void set_gram_rb(bool on) { g_gram_rb = on; g_rotate_rb = on; }
 
+// Splits of a Gram product that its consumer sums itself instead of a reduction
+// kernel (fold: the number of splits left in part, 0 when out holds the sum): a
+// launch less in each of two places of the chain of a small cell's step.
+constexpr int kFoldSplits = 16;
+
 template <typename R>
 // full: every element of S is consumed (the band Hamiltonian C^H H C with
 // band weights); otherwise the upper triangle suffices (W^H W is Hermitian,
@@ -1041,7 +1059,8 @@ template <typename R>
 // bands take the upper-tile kernel
 int launch_gram(int lx, const void* X0, const void* X1, int ly, const void* Y0, const void* Y1,
                 double2* part, double2* out, int nsk, int ng, int nb, int nsplit, cudaStream_t st,
-                int* flags, bool full) {
+                int* flags, bool full, int* fold) {
+  if (fold) *fold = 0;
   if (sizeof(R) == 4 && g_tc_mode == 2 && lx == ly) {   // tcgen05 Gram (TF32 x 3)
     const int ns = launch_gram_tc5(lx, X0, X1, Y0, Y1, part, nsk, ng, nb, nsplit, flags, st);
     if (ns < 0) return -ns;
@@ -1103,6 +1122,10 @@ int launch_gram(int lx, const void* X0, const void* X1, int ly, const void* Y0, 
     else
       return fail(JRG_ERR_INVALID, "launch_gram: unsupported layout pair");
     if (rc) return rc;
+    if (fold && sizeof(R) == 4 && g_tc_mode == 0 && nsplit <= kFoldSplits) {
+      *fold = nsplit;
+      return JRG_OK;
+    }
     const size_t n = (size_t)nsk * nb * nb;
     k_gram_reduce<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, out, nsplit, nb, nsk);
     JRG_LAUNCH_CHECK("k_gram_reduce");
@@ -1125,13 +1148,13 @@ int launch_gram(int lx, const void* X0, const void* X1, int ly, const void* Y0, 
 }
 
 int launch_cholesky_inv_df(const double2* S, double2* Ri, int nsk, int nb, int* flags, double min_pivot,
-                           cudaStream_t st);
+                           cudaStream_t st, int);
 // df: the FP32 path uses the double-float kernel (R itself is then not
 // written: only R^-1 is consumed)
 int launch_cholesky_inv(const double2* S, double2* Rm, double2* Ri, int nsk, int nb, int* flags,
-                        double* dinv_scratch, cudaStream_t st, double min_pivot, bool df) {
+                        double* dinv_scratch, cudaStream_t st, double min_pivot, bool df, int fold) {
   if (df && g_tc_mode == 0) {
-    const int r = launch_cholesky_inv_df(S, Ri, nsk, nb, flags, min_pivot, st);
+    const int r = launch_cholesky_inv_df(S, Ri, nsk, nb, flags, min_pivot, st, fold > 0 ? fold : 1);
     if (r < 0) return -r;
     if (r > 0) return JRG_OK;
   }
@@ -1145,10 +1168,10 @@ int launch_cholesky_inv(const double2* S, double2* Rm, double2* Ri, int nsk, int
 }
 
 int launch_adjoint_small(const double2* A, const double2* Ri, double2* Rh, double2* negM2, int nsk,
-                         int nb, cudaStream_t st, const double* f, double* eps) {
+                         int nb, cudaStream_t st, const double* f, double* eps, int fold) {
   const bool tiled = nb > 32;
   const unsigned parts = (unsigned)((nb * nb + kAdjSmallThreads - 1) / kAdjSmallThreads);
-  k_adjoint_small<<<dim3(nsk, parts), kAdjSmallThreads, 0, st>>>(A, Ri, Rh, negM2, nb, f, eps, !tiled);
+  k_adjoint_small<<<dim3(nsk, parts), kAdjSmallThreads, 0, st>>>(A, Ri, Rh, negM2, nb, f, eps, !tiled, fold);
   JRG_LAUNCH_CHECK("k_adjoint_small");
   if (tiled) {
     const unsigned nt = (unsigned)((nb + 31) / 32);
@@ -1466,7 +1489,7 @@ int launch_reorthonormalise(void* wr, void* wi, double2* scratch, int nsk, int n
   template int launch_unpack<R>(const void*, void*, void*, void*, int, int, int, double,          \
                                 cudaStream_t);                                                  \
   template int launch_gram<R>(int, const void*, const void*, int, const void*, const void*,       \
-                              double2*, double2*, int, int, int, int, cudaStream_t, int*, bool); \
+                              double2*, double2*, int, int, int, int, cudaStream_t, int*, bool, int*); \
   template int launch_rotate<R>(int, int, const void*, const void*, const double2*, const void*,  \
                                 const double2*, void*, void*, int, int, int, double, void*,     \
                                 cudaStream_t, int);

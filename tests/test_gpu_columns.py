@@ -130,3 +130,25 @@ def test_wave_grid_and_its_adjoint(shape, prec):
   adj = np.fft.fftn(g, axes=ax) / np.sqrt(37.5)
   for a, b in ((w.detach(), want), (c.grad, adj)):
     assert np.linalg.norm(a.cpu().numpy() - b) <= tol * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("nb", [1, 7, 8, 9, 16, 17, 24, 32])
+@pytest.mark.parametrize("grid,nk", [((16, 16, 16), 2), ((30, 24, 32), 3), ((40, 40, 40), 5)])
+def test_gram_splits_summed_by_their_consumers(grid, nk, nb):
+  """One to many G splits of the Gram products (summed in the Cholesky and adjoint
+  kernels while few): FP32 against the FP64 plan, at the FP32 path's tolerances."""
+  import torch
+  rng = np.random.default_rng(nb)
+  out = []
+  w = None
+  for prec in (64, 32):
+    plan = _plan(grid, nb, prec, nk=nk)
+    if w is None:
+      w = rng.standard_normal((2,) + plan.param_shape)
+    occ = np.full((1, nk, nb), 1.3 / nk)
+    x = torch.tensor(w, dtype=plan.rdtype, device="cuda")
+    e, gr, gi = plan.energy_and_grad(x[0], x[1], occ)
+    out.append((e[:5].cpu().numpy(), torch.stack([gr, gi]).double().cpu().numpy()))
+  (e64, g64), (e32, g32) = out
+  assert np.all(np.abs(e32 - e64) <= 2e-6 * np.maximum(np.abs(e64), 1.0))
+  assert np.abs(g32 - g64).max() <= 1e-4 * np.abs(g64).max()
