@@ -243,8 +243,8 @@ const char* jrg_last_error(void) { return g_err.c_str(); }
 
 int jrg_plan_destroy(jrg_plan* P) {
   if (!P) return JRG_OK;
-  void* ptrs[] = {P->d.gidx, P->d.sph_yz, P->d.plane_x, P->d.plane_off, P->d.row_off, P->d.rows,
-                  P->d.xact, P->d.tk, P->d.tkf, P->d.tw, P->d.vext, P->d.ginv, P->d.gvec, P->d.proj,
+  // gidx: the allocation of all small index tables
+  void* ptrs[] = {P->d.gidx, P->d.tk, P->d.tkf, P->d.tw, P->d.vext, P->d.ginv, P->d.gvec, P->d.proj,
                   P->d.rowmap, P->d.xmap, P->d.col_of};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -454,8 +454,21 @@ int jrg_plan_create(const jrg_plan_desc* d, jrg_plan** out) {
   int rc = JRG_OK;
 #define UP(field, vec) \
   if (!rc) rc = up((void**)&P->d.field, vec.data(), vec.size() * sizeof(vec[0]));
-  UP(gidx, gidx) UP(sph_yz, sph_yz) UP(plane_x, plane_x) UP(plane_off, plane_off)
-  UP(row_off, row_off) UP(rows, rows) UP(xact, xact) UP(tk, tk) UP(tkf, tkf)
+  {
+    // the small index tables in one allocation and one copy
+    std::vector<int> all;
+    std::vector<std::pair<int**, size_t>> at;
+    auto add = [&](int** field, const std::vector<int>& v) {
+      at.emplace_back(field, all.size());
+      all.insert(all.end(), v.begin(), v.end());
+    };
+    add(&P->d.gidx, gidx); add(&P->d.sph_yz, sph_yz); add(&P->d.plane_x, plane_x); add(&P->d.plane_off, plane_off);
+    add(&P->d.row_off, row_off); add(&P->d.rows, rows); add(&P->d.xact, xact);
+    rc = up((void**)&P->d.gidx, all.data(), all.size() * sizeof(int));
+    if (!rc)
+      for (auto& f : at) *f.first = P->d.gidx + f.second;   // gidx itself stands first
+  }
+  UP(tk, tk) UP(tkf, tkf)
   if (P->cols) {
     UP(xmap, xmap) UP(col_of, col_of)
   } else {
