@@ -338,11 +338,13 @@ int jrg_precond_scale(const jrg_plan* plan, const float* w32, const void* wb, fl
 int jrg_band_kinetic(const jrg_plan* plan, const void* workspace, double* out, cudaStream_t stream);
 int jrg_kinetic_table(const jrg_plan* plan, double* out, cudaStream_t stream);
 
-/* Selects the specialised kernels (enable = 1, the default): register-
- * resident slab FFTs for cubic grids N^3 with N in {16, 24, 27, 32, 36, 48,
- * 64, 96} and register-blocked Gram contractions for num_band <= 32; or the
- * generic ones (enable = 0): shared-memory Stockham FFTs for every grid and
- * 32x32-tiled Gram contractions.  enable < 0 only queries.  Returns the
+/* Selects the specialised kernels (enable = 1, the default): column-first
+ * transforms for spheres in the alias-free window |i| < N/4 of every axis,
+ * each axis one of the 7-smooth lengths 16 to 96 but 75 and 81 (FP64: not
+ * 32^3 and 64^3); register-resident slab FFTs for other spheres on cubic grids
+ * N^3 with N in {16, 24, 27, 32, 36, 48, 64, 96}; and register-blocked Gram
+ * contractions for num_band <= 32; or the generic ones (enable = 0): shared-
+ * memory Stockham FFTs for every grid and 32x32-tiled Gram contractions.  enable < 0 only queries.  Returns the
  * previous setting.  Process-wide; no reference counterpart. */
 int jrg_fast_paths(int enable);
 
@@ -363,7 +365,8 @@ int jrg_tensor_core_paths(int enable);
  * halves that run on the caller's stream and a second stream owned by the
  * plan (joined back before the call returns, in stream order), so that the
  * latency-bound small kernels of one half overlap the other half's
- * bandwidth-bound kernels.  enable = 0 runs everything on the caller's
+ * bandwidth-bound kernels; sums that only the energies need run on a third
+ * stream beside them.  enable = 0 runs everything on the caller's
  * stream; < 0 only queries.  Returns the previous setting.  Process-wide; no
  * reference counterpart. */
 int jrg_pipeline(int enable);

@@ -64,11 +64,13 @@ __device__ __forceinline__ void rg_load(const void* __restrict__ a, const void* 
 }
 
 // Accumulators of TG G vectors x NJ columns and acc[q][jj] += x[q] * M[row][jj].
-// FP32: packed over pairs of columns (fma.rn.f32x2: the FP32 pipe's rate at half
-// the issue slots), M staged as (re, re', im, im') of a pair, one 16-byte load.
-// Scalar before: adjoint and Adam 240 us, packed 220 (Si8, 24 bands); 160 bands:
-// forward 1.64 and 1.57 ms, adjoint and Adam 4.55 and 4.47 ms.
-template <typename R, int NJ, int TG> struct RgAcc {
+// FP32 tiles of 32 columns are packed over pairs of columns (fma.rn.f32x2: the FP32
+// pipe's rate at half the issue slots), M staged as (re, re', im, im') of a pair,
+// one 16-byte load: at 160 bands forward 1.64 -> 1.57 ms, adjoint 3.80 -> 3.51.
+// Narrower tiles wait for memory more than for issue slots: 24 bands, adjoint 111
+// us scalar and 119 packed.
+template <int NJ> __host__ __device__ constexpr bool rg_packed() { return NJ >= 32; }
+template <typename R, int NJ, int TG, bool PACKED = sizeof(R) == 4 && rg_packed<NJ>()> struct RgAcc {
   C_t<R> v[TG][NJ];
   __device__ __forceinline__ void zero() {
 #pragma unroll
@@ -77,6 +79,20 @@ template <typename R, int NJ, int TG> struct RgAcc {
       for (int jj = 0; jj < NJ; ++jj) v[q][jj] = czero<C_t<R>>();
   }
   __device__ __forceinline__ void row(const C_t<R> (&x)[TG], const C_t<R>* __restrict__ mrow) {
+    if constexpr (sizeof(R) == 4) {
+#pragma unroll
+      for (int jj = 0; jj < NJ; jj += 2) {
+        const float4 m = *reinterpret_cast<const float4*>(mrow + jj);
+#pragma unroll
+        for (int q = 0; q < TG; ++q) {
+          v[q][jj].x = fmaf(x[q].x, m.x, fmaf(-x[q].y, m.y, v[q][jj].x));
+          v[q][jj].y = fmaf(x[q].x, m.y, fmaf(x[q].y, m.x, v[q][jj].y));
+          v[q][jj + 1].x = fmaf(x[q].x, m.z, fmaf(-x[q].y, m.w, v[q][jj + 1].x));
+          v[q][jj + 1].y = fmaf(x[q].x, m.w, fmaf(x[q].y, m.z, v[q][jj + 1].y));
+        }
+      }
+      return;
+    }
 #pragma unroll
     for (int jj = 0; jj < NJ; ++jj) {
       const C_t<R> m = mrow[jj];
@@ -90,7 +106,7 @@ template <typename R, int NJ, int TG> struct RgAcc {
   __device__ __forceinline__ C_t<R> get(int q, int jj) const { return v[q][jj]; }
   static __device__ __forceinline__ void stage(C_t<R>* ms, int e, double2 m) { ms[e] = cmk<C_t<R>>(m.x, m.y); }
 };
-template <int NJ, int TG> struct RgAcc<float, NJ, TG> {
+template <int NJ, int TG> struct RgAcc<float, NJ, TG, true> {
   static_assert(NJ % 2 == 0, "column pairs");
   float2 re[TG][NJ / 2], im[TG][NJ / 2];
   __device__ __forceinline__ void zero() {
