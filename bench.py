@@ -279,11 +279,11 @@ def _config(wl, n, precision=None):
           "l2": "no explicit flush: each step streams >0.9 GB of columns, coefficients and parameters, >7x the 129 MB L2"}
 
 
-# DRAM bytes (read + write) per band of one k_line_apply_v<float, 64> launch,
-# from an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum) of the
-# 64^3 Si8 cell at 2x2x2 k-points (135 MB for the 96 bands of one pipeline
-# half); a full launch is scaled by its band count
-LINE_APPLY_V_DRAM_PER_BAND = (98.57996e6 + 36.56985e6) / 96
+# DRAM bytes (read + write) per occupied band of one k_cube_apply_v<float, 64>
+# launch, from an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum) of
+# the 64^3 Si8 cell at 2x2x2 k-points (27.1 MB for the 64 occupied bands of one
+# pipeline half; the results stay in L2); a full launch is scaled by its band count
+LINE_APPLY_V_DRAM_PER_BAND = 27.1e6 / 64
 
 
 # algorithmic bytes per call of each phase of jrg_energy_grad (fused: the

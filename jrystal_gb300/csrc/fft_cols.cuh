@@ -16,8 +16,8 @@
 //
 // Before, the planes of each band were transformed in y and z first, by several
 // threads a line with a shared-memory exchange in every transform: 0.99 ms for the
-// four passes at the Si8 64^3 workload (27 k-points, 24 bands, FP32), now 0.56 ms;
-// at 96^3 (160 bands) 12.9, now 8.4 ms; 30 x 45 x 64 (84 bands) 444, now 145 us.
+// four passes at the Si8 64^3 workload (27 k-points, 24 bands, FP32), now 0.55 ms;
+// at 96^3 (160 bands) 12.9, now 6.4 ms; 30 x 45 x 64 (84 bands) 444, now 146 us.
 //
 // Every active index of the sphere lies in the alias-free window |i| < N/4 of its
 // axis; spheres that reach further keep the plane-first kernels (k_fft_fast.cu,
