@@ -33,7 +33,7 @@ namespace jrg {
 
 template <typename R>
 int launch_adam(void*, const void*, void*, void*, const float*, long long, double, double, double, double,
-                double, double, cudaStream_t, const int*, const double*);
+                double, cudaStream_t, const int*, const double*);
 
 struct BatchCell {
   const void* params;       // [2][n] in the cell's precision
@@ -192,10 +192,10 @@ static int batch_enqueue(jrg_batch* b, cudaStream_t st) {
     else k_batch_record<float><<<1, kRecThreads, 0, s>>>(b->cells[c]);
     JRG_LAUNCH_CHECK("k_batch_record");
     const int* guard = (const int*)((const char*)b->ws[c] + P->ws.flags);
-    rc = P->prec == 64 ? launch_adam<double>(pr, gr, b->m[c], b->v[c], nullptr, 2 * b->cells[c].n, b->lr, b->b1,
-                                             b->b2, 1.0, 1.0, b->eps, s, guard, b->cells[c].coef_cur)
-                       : launch_adam<float>(pr, gr, b->m[c], b->v[c], nullptr, 2 * b->cells[c].n, b->lr, b->b1,
-                                            b->b2, 1.0, 1.0, b->eps, s, guard, b->cells[c].coef_cur);
+    rc = P->prec == 64 ? launch_adam<double>(pr, gr, b->m[c], b->v[c], nullptr, 2 * b->cells[c].n, 0.0, b->b1,
+                                             b->b2, 0.0, b->eps, s, guard, b->cells[c].coef_cur)
+                       : launch_adam<float>(pr, gr, b->m[c], b->v[c], nullptr, 2 * b->cells[c].n, 0.0, b->b1,
+                                            b->b2, 0.0, b->eps, s, guard, b->cells[c].coef_cur);
     if (rc) return rc;
     JRG_CUDA(cudaEventRecord(b->done[c], s));
     JRG_CUDA(cudaStreamWaitEvent(st, b->done[c], 0));
@@ -248,8 +248,8 @@ int jrg_batch_create(const jrg_batch_desc* d, jrg_batch** out) {
   // prev_idx, prev_g, prev_p
   std::vector<double> tab(2 * (size_t)T);
   for (int t = 0; t < T; ++t) {
-    tab[2 * t] = 1.0 - std::pow(d->b1, t + 1);
-    tab[2 * t + 1] = 1.0 - std::pow(d->b2, t + 1);
+    tab[2 * t] = -d->lr / (1.0 - std::pow(d->b1, t + 1));
+    tab[2 * t + 1] = 1.0 / (1.0 - std::pow(d->b2, t + 1));
   }
   const size_t tab_bytes = tab.size() * sizeof(double);
   const size_t per_cell = 8 * sizeof(double) + 2 * sizeof(double) + (size_t)P * sizeof(long long) +

@@ -60,7 +60,7 @@ template <typename R> int launch_potential_gga(const void*, double, void*, const
 constexpr int kXcGga = JRG_XC_GGA_X_PBE | JRG_XC_GGA_C_PBE;
 template <typename R> int launch_geometry_tables(double*, double*, void*, double2*, const double*, const double*, const double*, int, int, int, int, double, cudaStream_t);
 int launch_ewald(const double*, const double*, const double*, const double*, int, int, long long, double, double, double*, int, double*, cudaStream_t);
-template <typename R> int launch_adam(void*, const void*, void*, void*, const float*, long long, double, double, double, double, double, double, cudaStream_t, const int* = nullptr, const double* = nullptr);
+template <typename R> int launch_adam(void*, const void*, void*, void*, const float*, long long, double, double, double, double, double, cudaStream_t, const int* = nullptr, const double* = nullptr);
 int launch_twiddles(int n, int prec, void* out, cudaStream_t st);
 template <typename R> int launch_reorthonormalise(void*, void*, double2*, int, int, int, cudaStream_t);
 int launch_dft_axis_inv_f64(const double2*, double2*, int, int, int, int, const double2*, cudaStream_t);
@@ -1396,9 +1396,9 @@ int jrg_energy_grad_adam(const jrg_plan* P, void* params, void* m, void* v, cons
   a.v[0] = v; a.v[1] = hi(v);
   a.scale[0] = opt->scale; a.scale[1] = opt->scale ? opt->scale + n : nullptr;
   a.grad[0] = grad; a.grad[1] = hi(grad);
-  a.lr = opt->lr; a.b1 = opt->b1; a.b2 = opt->b2; a.eps = opt->eps;
-  a.c1 = 1.0 - std::pow(opt->b1, opt->step);
-  a.c2 = 1.0 - std::pow(opt->b2, opt->step);
+  a.b1 = opt->b1; a.b2 = opt->b2; a.eps = opt->eps;
+  a.up = -opt->lr / (1.0 - std::pow(opt->b1, opt->step));
+  a.iv = 1.0 / (1.0 - std::pow(opt->b2, opt->step));
   a.mlp_w32 = opt->mlp_w32; a.mlp_wb = opt->mlp_wb;
   a.t_frac = opt->t_frac; a.smax = opt->smax;
   a.guard = (const int*)((const char*)ws + P->ws.flags);
@@ -1524,9 +1524,9 @@ int jrg_adam_update(int prec, int64_t n, void* param, const void* grad, void* m,
                     cudaStream_t st) {
   if (!param || !grad || !m || !v || n < 0 || step < 1 || (prec != 32 && prec != 64))
     return fail(JRG_ERR_INVALID, "jrg_adam_update: bad argument");
-  const double c1 = 1.0 - std::pow(b1, step), c2 = 1.0 - std::pow(b2, step);
-  if (prec == 64) return launch_adam<double>(param, grad, m, v, scale, n, lr, b1, b2, c1, c2, eps, st);
-  return launch_adam<float>(param, grad, m, v, scale, n, lr, b1, b2, c1, c2, eps, st);
+  const double up = -lr / (1.0 - std::pow(b1, step)), iv = 1.0 / (1.0 - std::pow(b2, step));
+  if (prec == 64) return launch_adam<double>(param, grad, m, v, scale, n, up, b1, b2, iv, eps, st);
+  return launch_adam<float>(param, grad, m, v, scale, n, up, b1, b2, iv, eps, st);
 }
 
 int jrg_ewald(const jrg_plan* P, double eta, double cutoff, double* result, void* ws, cudaStream_t st) {

@@ -936,58 +936,72 @@ __global__ void k_ewald_finish(const double* __restrict__ slots, int nslots, con
 // Adam (optax placement of eps) with optional elementwise update scale
 // ------------------------------------------------------------------------
 
-template <typename R>
+// U 16-byte groups of each array per thread and pass, all loaded before the
+// arithmetic.  Bound by HBM (four arrays read, three written).  The moments of empty
+// bands are zero, and a division of zero takes the division's slow path: with the two
+// bias corrections as factors one division per element is left of three.  2 x 5.7M
+// FP32 elements, a third of them zero: 81 us with three divisions and one group, 58
+// with one division, 56 (5.8 TB/s) with two groups; no zeros 56, 55, 52.
+// 2 x 46M: 584, 420, 386 and 400, 390, 369.
+template <typename R, int U>
 __device__ __forceinline__ void adam_range(R* __restrict__ p, const R* __restrict__ g, R* __restrict__ m,
-                       R* __restrict__ v, const float* __restrict__ scale, long long n, R lr, R b1,
-                       R b2, R c1, R c2, R eps, const int* __restrict__ guard,
-                       const double* __restrict__ coefs) {
+                       R* __restrict__ v, const float* __restrict__ scale, long long n, R up, R b1,
+                       R b2, R iv, R eps, const int* __restrict__ guard, const double* __restrict__ coefs) {
   // guard: the status word of the energy call that made g; non-zero (a
   // Cholesky breakdown) leaves the parameters and moments unchanged
   if (guard && *guard) return;
-  // coefs: bias corrections (c1, c2) read from device memory instead of the
-  // arguments (a step replayed from a CUDA graph, the step count on device)
-  if (coefs) { c1 = (R)coefs[0]; c2 = (R)coefs[1]; }
+  // coefs: (up, iv) read from device memory instead of the arguments (a step
+  // replayed from a CUDA graph, the step count on device)
+  if (coefs) { up = (R)coefs[0]; iv = (R)coefs[1]; }
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  long long done = 0;
   if constexpr (sizeof(R) == 4) {
-    // four elements per thread with 16-byte accesses when the buffers are aligned
+    // 16-byte accesses when the buffers are aligned
     const bool vec = (((uintptr_t)p | (uintptr_t)g | (uintptr_t)m | (uintptr_t)v |
                        (uintptr_t)scale) & 15) == 0;
     const long long n4 = vec ? n / 4 : 0;
-    for (long long q = tid; q < n4; q += stride) {
-      float4 pp = reinterpret_cast<float4*>(p)[q];
-      const float4 gg = reinterpret_cast<const float4*>(g)[q];
-      float4 mm = reinterpret_cast<float4*>(m)[q];
-      float4 vv = reinterpret_cast<float4*>(v)[q];
-      float4 u;
-      u.x = adam_one<float>(gg.x, mm.x, vv.x, lr, b1, b2, c1, c2, eps);
-      u.y = adam_one<float>(gg.y, mm.y, vv.y, lr, b1, b2, c1, c2, eps);
-      u.z = adam_one<float>(gg.z, mm.z, vv.z, lr, b1, b2, c1, c2, eps);
-      u.w = adam_one<float>(gg.w, mm.w, vv.w, lr, b1, b2, c1, c2, eps);
-      if (scale) {
-        const float4 s = reinterpret_cast<const float4*>(scale)[q];
-        u.x *= s.x; u.y *= s.y; u.z *= s.z; u.w *= s.w;
+    done = 4 * n4;
+    const long long first = blockIdx.x * (long long)(U * blockDim.x) + threadIdx.x;
+    for (long long q0 = first; q0 < n4; q0 += U * stride) {
+      float4 pp[U], gg[U], mm[U], vv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long q = q0 + u * blockDim.x;
+        if (q < n4) {
+          pp[u] = reinterpret_cast<float4*>(p)[q];
+          gg[u] = reinterpret_cast<const float4*>(g)[q];
+          mm[u] = reinterpret_cast<float4*>(m)[q];
+          vv[u] = reinterpret_cast<float4*>(v)[q];
+        }
       }
-      pp.x += u.x; pp.y += u.y; pp.z += u.z; pp.w += u.w;
-      reinterpret_cast<float4*>(p)[q] = pp;
-      reinterpret_cast<float4*>(m)[q] = mm;
-      reinterpret_cast<float4*>(v)[q] = vv;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long q = q0 + u * blockDim.x;
+        if (q < n4) {
+          float4 d;
+          d.x = adam_one<float>(gg[u].x, mm[u].x, vv[u].x, up, b1, b2, iv, eps);
+          d.y = adam_one<float>(gg[u].y, mm[u].y, vv[u].y, up, b1, b2, iv, eps);
+          d.z = adam_one<float>(gg[u].z, mm[u].z, vv[u].z, up, b1, b2, iv, eps);
+          d.w = adam_one<float>(gg[u].w, mm[u].w, vv[u].w, up, b1, b2, iv, eps);
+          if (scale) {
+            const float4 s = reinterpret_cast<const float4*>(scale)[q];
+            d.x *= s.x; d.y *= s.y; d.z *= s.z; d.w *= s.w;
+          }
+          pp[u].x += d.x; pp[u].y += d.y; pp[u].z += d.z; pp[u].w += d.w;
+          reinterpret_cast<float4*>(p)[q] = pp[u];
+          reinterpret_cast<float4*>(m)[q] = mm[u];
+          reinterpret_cast<float4*>(v)[q] = vv[u];
+        }
+      }
     }
-    for (long long i = 4 * n4 + tid; i < n; i += stride) {
-      R mi = m[i], vi = v[i];
-      R u = adam_one<R>(g[i], mi, vi, lr, b1, b2, c1, c2, eps);
-      m[i] = mi; v[i] = vi;
-      if (scale) u *= (R)scale[i];
-      p[i] += u;
-    }
-  } else {
-    for (long long i = tid; i < n; i += stride) {
-      R mi = m[i], vi = v[i];
-      R u = adam_one<R>(g[i], mi, vi, lr, b1, b2, c1, c2, eps);
-      m[i] = mi; v[i] = vi;
-      if (scale) u *= (R)scale[i];
-      p[i] += u;
-    }
+  }
+  for (long long i = done + tid; i < n; i += stride) {
+    R mi = m[i], vi = v[i];
+    R d = adam_one<R>(g[i], mi, vi, up, b1, b2, iv, eps);
+    m[i] = mi; v[i] = vi;
+    if (scale) d *= (R)scale[i];
+    p[i] += d;
   }
 }
 
@@ -1033,11 +1047,12 @@ __global__ void k_twiddles(int n, C_t<R>* __restrict__ out) {
   }
 }
 
-template <typename R>
-__global__ void k_adam(R* __restrict__ p, const R* __restrict__ g, R* __restrict__ m, R* __restrict__ v,
-                       const float* __restrict__ scale, long long n, R lr, R b1, R b2, R c1, R c2, R eps,
-                       const int* __restrict__ guard, const double* __restrict__ coefs) {
-  adam_range<R>(p, g, m, v, scale, n, lr, b1, b2, c1, c2, eps, guard, coefs);
+template <typename R, int U>
+__global__ void __launch_bounds__(256)
+k_adam(R* __restrict__ p, const R* __restrict__ g, R* __restrict__ m, R* __restrict__ v,
+       const float* __restrict__ scale, long long n, R up, R b1, R b2, R iv, R eps,
+       const int* __restrict__ guard, const double* __restrict__ coefs) {
+  adam_range<R, U>(p, g, m, v, scale, n, up, b1, b2, iv, eps, guard, coefs);
 }
 
 // real and imaginary parts in one launch (blockIdx.y): the optimiser step of a
@@ -1045,11 +1060,11 @@ __global__ void k_adam(R* __restrict__ p, const R* __restrict__ g, R* __restrict
 template <typename R> struct AdamPair {
   R* p[2]; const R* g[2]; R* m[2]; R* v[2]; const float* scale[2];
 };
-template <typename R>
-__global__ void k_adam_pair(AdamPair<R> a, long long n, R lr, R b1, R b2, R c1, R c2, R eps,
-                            const int* __restrict__ guard) {
+template <typename R, int U>
+__global__ void __launch_bounds__(256)
+k_adam_pair(AdamPair<R> a, long long n, R up, R b1, R b2, R iv, R eps, const int* __restrict__ guard) {
   const int q = blockIdx.y;
-  adam_range<R>(a.p[q], a.g[q], a.m[q], a.v[q], a.scale[q], n, lr, b1, b2, c1, c2, eps, guard, nullptr);
+  adam_range<R, U>(a.p[q], a.g[q], a.m[q], a.v[q], a.scale[q], n, up, b1, b2, iv, eps, guard, nullptr);
 }
 
 // ------------------------------------------------------------------------
@@ -1262,8 +1277,13 @@ int launch_adam_pair(const AdamArgs& a, size_t off, const void* g0, const void* 
     q.g[part] = reinterpret_cast<const R*>(part ? g1 : g0);
     q.scale[part] = a.scale[part] ? a.scale[part] + off : nullptr;
   }
-  k_adam_pair<R><<<dim3(grid_for((n + 3) / 4, 256, 152 * 8), 2), 256, 0, st>>>(q, n, (R)a.lr, (R)a.b1, (R)a.b2, (R)a.c1,
-                                                                    (R)a.c2, (R)a.eps, a.guard);
+  // two groups per thread once one would need more CTAs than the SMs hold at a
+  // time (2 x 262K elements, 512 CTAs, a third zeros: 7.0 us with one, 7.8 with two)
+  const unsigned one = grid_for((n + 3) / 4, 256, 1 << 30);
+  if (sizeof(R) == 4 && 2LL * one > 152 * 8)
+    k_adam_pair<R, 2><<<dim3((one + 1) / 2, 2), 256, 0, st>>>(q, n, (R)a.up, (R)a.b1, (R)a.b2, (R)a.iv, (R)a.eps, a.guard);
+  else
+    k_adam_pair<R, 1><<<dim3(one, 2), 256, 0, st>>>(q, n, (R)a.up, (R)a.b1, (R)a.b2, (R)a.iv, (R)a.eps, a.guard);
   JRG_LAUNCH_CHECK("k_adam_pair");
   return JRG_OK;
 }
@@ -1271,12 +1291,16 @@ template int launch_adam_pair<float>(const AdamArgs&, size_t, const void*, const
 template int launch_adam_pair<double>(const AdamArgs&, size_t, const void*, const void*, long long, cudaStream_t);
 
 template <typename R>
-int launch_adam(void* p, const void* g, void* m, void* v, const float* scale, long long n, double lr,
-                double b1, double b2, double c1, double c2, double eps, cudaStream_t st,
+int launch_adam(void* p, const void* g, void* m, void* v, const float* scale, long long n, double up,
+                double b1, double b2, double iv, double eps, cudaStream_t st,
                 const int* guard, const double* coefs) {
-  k_adam<R><<<grid_for((n + 3) / 4, 256, 152 * 16), 256, 0, st>>>(
-      reinterpret_cast<R*>(p), reinterpret_cast<const R*>(g), reinterpret_cast<R*>(m),
-      reinterpret_cast<R*>(v), scale, n, (R)lr, (R)b1, (R)b2, (R)c1, (R)c2, (R)eps, guard, coefs);
+  const unsigned one = grid_for((n + 3) / 4, 256, 1 << 30);
+  auto go = [&](auto kernel, unsigned blocks) {
+    kernel<<<blocks, 256, 0, st>>>(reinterpret_cast<R*>(p), reinterpret_cast<const R*>(g), reinterpret_cast<R*>(m),
+                                   reinterpret_cast<R*>(v), scale, n, (R)up, (R)b1, (R)b2, (R)iv, (R)eps, guard, coefs);
+  };
+  if (sizeof(R) == 4 && one > 152 * 8) go(k_adam<R, 2>, (one + 1) / 2);   // as launch_adam_pair
+  else go(k_adam<R, 1>, one);
   JRG_LAUNCH_CHECK("k_adam");
   return JRG_OK;
 }
@@ -1328,7 +1352,7 @@ int launch_twiddles(int n, int prec, void* out, cudaStream_t st) {
   template int launch_potential_gga<R>(const void*, double, void*, const void*, long long,        \
                                        const double*, cudaStream_t);                            \
   template int launch_adam<R>(void*, const void*, void*, void*, const float*, long long, double,  \
-                              double, double, double, double, double, cudaStream_t, const int*,  \
+                              double, double, double, double, cudaStream_t, const int*,          \
                               const double*);
 JRG_INST_GRID(float)
 JRG_INST_GRID(double)

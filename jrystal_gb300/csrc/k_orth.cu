@@ -953,8 +953,7 @@ k_rotate_rb(const void* __restrict__ X0a, const void* __restrict__ X0b, const do
     // a Cholesky breakdown of this call leaves parameters and moments as they
     // were (the flag is final: every Cholesky of the call ran before)
     if (adam.guard && *adam.guard) return;
-    const R lr = (R)adam.lr, b1 = (R)adam.b1, b2 = (R)adam.b2, c1 = (R)adam.c1, c2 = (R)adam.c2,
-            eps = (R)adam.eps;
+    const R up = (R)adam.up, b1 = (R)adam.b1, b2 = (R)adam.b2, iv = (R)adam.iv, eps = (R)adam.eps;
     constexpr int U = 8;
     for (int e0 = t; e0 < 2 * len; e0 += U * 256) {
       R mi[U], vi[U], pi[U];
@@ -978,7 +977,7 @@ k_rotate_rb(const void* __restrict__ X0a, const void* __restrict__ X0b, const do
           const int r = el / nb;
           const R gr = tile[(part * GT + r) * (NBP + 1) + (el - r * nb)];
           if (adam.grad[part]) reinterpret_cast<R*>(adam.grad[part])[base + el] = gr;
-          R d = adam_one<R>(gr, mi[u], vi[u], lr, b1, b2, c1, c2, eps);
+          R d = adam_one<R>(gr, mi[u], vi[u], up, b1, b2, iv, eps);
           if (adam.scale[part]) d *= (R)si[u];
           reinterpret_cast<R*>(adam.m[part])[base + el] = mi[u];
           reinterpret_cast<R*>(adam.v[part])[base + el] = vi[u];

@@ -292,8 +292,7 @@ k_rotate_g(const void* __restrict__ X0a, const void* __restrict__ X0b, const dou
     // Adam on this thread's elements of the tile (both parts); a Cholesky
     // breakdown of the call (status word non-zero) leaves everything as it was
     if (adam.guard && *adam.guard) return;
-    const R lr = (R)adam.lr, b1 = (R)adam.b1, b2 = (R)adam.b2, c1 = (R)adam.c1, c2 = (R)adam.c2,
-            eps = (R)adam.eps;
+    const R up = (R)adam.up, b1 = (R)adam.b1, b2 = (R)adam.b2, iv = (R)adam.iv, eps = (R)adam.eps;
 #pragma unroll
     for (int q = 0; q < TG; ++q) {
       if (g[q] >= ng) continue;
@@ -319,7 +318,7 @@ k_rotate_g(const void* __restrict__ X0a, const void* __restrict__ X0b, const dou
               if (sc) *reinterpret_cast<float4*>(sv) = *reinterpret_cast<const float4*>(sc + jj);
               if (gout) *reinterpret_cast<float4*>(gout + jj) = *reinterpret_cast<const float4*>(gv);
 #pragma unroll
-              for (int u = 0; u < 4; ++u) pv[u] += sv[u] * adam_one<float>(gv[u], mv[u], vv[u], lr, b1, b2, c1, c2, eps);
+              for (int u = 0; u < 4; ++u) pv[u] += sv[u] * adam_one<float>(gv[u], mv[u], vv[u], up, b1, b2, iv, eps);
               *reinterpret_cast<float4*>(m + jj) = *reinterpret_cast<const float4*>(mv);
               *reinterpret_cast<float4*>(v + jj) = *reinterpret_cast<const float4*>(vv);
               *reinterpret_cast<float4*>(p + jj) = *reinterpret_cast<const float4*>(pv);
@@ -340,7 +339,7 @@ k_rotate_g(const void* __restrict__ X0a, const void* __restrict__ X0b, const dou
             const R gr = fac * (part ? acc[q][jj].y : acc[q][jj].x);
             if (gout) gout[jj] = gr;
             R mi = m[jj], vi = v[jj];
-            R d = adam_one<R>(gr, mi, vi, lr, b1, b2, c1, c2, eps);
+            R d = adam_one<R>(gr, mi, vi, up, b1, b2, iv, eps);
             if (sc) d *= (R)sc[jj];
             m[jj] = mi;
             v[jj] = vi;

@@ -97,7 +97,8 @@ struct AdamArgs {
   void* v[2];
   float* scale[2];        // per-element update scale (optional; learned scales when mlp_w32)
   void* grad[2];          // gradient output (optional)
-  double lr, b1, b2, c1, c2, eps;
+  double up, iv;          // -lr / (1 - b1^t), 1 / (1 - b2^t)
+  double b1, b2, eps;
   const float* mlp_w32;   // learned preconditioner evaluated inside the step (optional)
   const void* mlp_wb;
   float t_frac, smax;
