@@ -1063,8 +1063,9 @@ template <typename R> struct AdamPair {
 template <typename R, int U>
 __global__ void __launch_bounds__(256)
 k_adam_pair(AdamPair<R> a, long long n, R up, R b1, R b2, R iv, R eps, const int* __restrict__ guard) {
-  const int q = blockIdx.y;
-  adam_range<R, U>(a.p[q], a.g[q], a.m[q], a.v[q], a.scale[q], n, up, b1, b2, iv, eps, guard, nullptr);
+  const bool q = blockIdx.y;      // selected, not indexed: an indexed argument is copied to local memory
+  adam_range<R, U>(q ? a.p[1] : a.p[0], q ? a.g[1] : a.g[0], q ? a.m[1] : a.m[0], q ? a.v[1] : a.v[0],
+                   q ? a.scale[1] : a.scale[0], n, up, b1, b2, iv, eps, guard, nullptr);
 }
 
 // ------------------------------------------------------------------------
@@ -1280,8 +1281,9 @@ int launch_adam_pair(const AdamArgs& a, size_t off, const void* g0, const void* 
   // two groups per thread once one would need more CTAs than the SMs hold at a
   // time (2 x 262K elements, 512 CTAs, a third zeros: 7.0 us with one, 7.8 with two)
   const unsigned one = grid_for((n + 3) / 4, 256, 1 << 30);
-  if (sizeof(R) == 4 && 2LL * one > 152 * 8)
-    k_adam_pair<R, 2><<<dim3((one + 1) / 2, 2), 256, 0, st>>>(q, n, (R)a.up, (R)a.b1, (R)a.b2, (R)a.iv, (R)a.eps, a.guard);
+  constexpr int U = sizeof(R) == 4 ? 2 : 1;
+  if (2LL * one > 152 * 8)
+    k_adam_pair<R, U><<<dim3((one + U - 1) / U, 2), 256, 0, st>>>(q, n, (R)a.up, (R)a.b1, (R)a.b2, (R)a.iv, (R)a.eps, a.guard);
   else
     k_adam_pair<R, 1><<<dim3(one, 2), 256, 0, st>>>(q, n, (R)a.up, (R)a.b1, (R)a.b2, (R)a.iv, (R)a.eps, a.guard);
   JRG_LAUNCH_CHECK("k_adam_pair");
@@ -1299,7 +1301,8 @@ int launch_adam(void* p, const void* g, void* m, void* v, const float* scale, lo
     kernel<<<blocks, 256, 0, st>>>(reinterpret_cast<R*>(p), reinterpret_cast<const R*>(g), reinterpret_cast<R*>(m),
                                    reinterpret_cast<R*>(v), scale, n, (R)up, (R)b1, (R)b2, (R)iv, (R)eps, guard, coefs);
   };
-  if (sizeof(R) == 4 && one > 152 * 8) go(k_adam<R, 2>, (one + 1) / 2);   // as launch_adam_pair
+  constexpr int U = sizeof(R) == 4 ? 2 : 1;
+  if (one > 152 * 8) go(k_adam<R, U>, (one + U - 1) / U);   // as launch_adam_pair
   else go(k_adam<R, 1>, one);
   JRG_LAUNCH_CHECK("k_adam");
   return JRG_OK;
