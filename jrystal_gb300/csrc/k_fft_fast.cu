@@ -753,14 +753,15 @@ __global__ void __launch_bounds__(hartree_threads<N>()) k_line_hartree(
   __syncthreads();
   if (act) reg::line_step_a<N, -1>(v, tw, j2, ex, L, zl);
   __syncthreads();
+  const double sn = s * inv_n;
   double eh = 0.0;
   if (act) {
     reg::line_step_b<N, -1>(v, j2, ex, L, zl);
 #pragma unroll
     for (int j = 0; j < N1; ++j) {
       const double gi = ginv[((size_t)(N2 * j + j2) * N + y) * N + z];
-      const double rx = v[j].x, ry = v[j].y, t = s * gi * inv_n;
-      eh += 0.5 * gi * (rx * rx + ry * ry);
+      const double rx = v[j].x, ry = v[j].y, t = sn * gi;
+      eh += gi * (rx * rx + ry * ry);
       v[j].x = (R)(t * rx);
       v[j].y = (R)(t * ry);
     }
@@ -774,7 +775,7 @@ __global__ void __launch_bounds__(hartree_threads<N>()) k_line_hartree(
     for (int j = 0; j < N1; ++j) line[(size_t)(N2 * j + j2) * (N * N)] = v[j];
   }
   eh = block_sum(eh, red);
-  if (tid == 0) slot_h[cta] = eh * pref * s * s;
+  if (tid == 0) slot_h[cta] = 0.5 * eh * pref * s * s;
   if (cta == 0)
     for (int i = nctas + tid; i < nslots; i += blockDim.x) slot_h[i] = 0.0;
 }

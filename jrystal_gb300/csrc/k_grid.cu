@@ -432,11 +432,10 @@ __global__ void __launch_bounds__(kGridThreads) k_potential_pol(const R* __restr
     vr[i] = (R)(base + rt * du);
     vr[ngrid + i] = (R)(base + rt * dd);
   }
-  ex = block_sum(ex, red);
-  if (threadIdx.x == 0) slot_x[blockIdx.x] = ex * pref;
-  if (slot_e) {
-    ee = block_sum(ee, red);
-    if (threadIdx.x == 0) slot_e[blockIdx.x] = ee * pref;
+  block_sum2(ex, ee, red);
+  if (threadIdx.x == 0) {
+    slot_x[blockIdx.x] = ex * pref;
+    if (slot_e) slot_e[blockIdx.x] = ee * pref;
   }
 }
 
@@ -653,11 +652,10 @@ __global__ void __launch_bounds__(kGridThreads, 4) k_potential(const R* __restri
     }
     if (vr) vr[i] = (R)((double)vri[i].x * vscale + v + ve);
   }
-  ex = block_sum(ex, red);
-  if (threadIdx.x == 0) slot_x[blockIdx.x] = ex * pref;
-  if (slot_e) {
-    ee = block_sum(ee, red);
-    if (threadIdx.x == 0) slot_e[blockIdx.x] = ee * pref;
+  block_sum2(ex, ee, red);
+  if (threadIdx.x == 0) {
+    slot_x[blockIdx.x] = ex * pref;
+    if (slot_e) slot_e[blockIdx.x] = ee * pref;
   }
 }
 
