@@ -23,6 +23,12 @@ def _ptr(t: Optional[torch.Tensor]):
   return None if t is None else ct.c_void_p(t.data_ptr())
 
 
+def _plain(t: torch.Tensor) -> torch.Tensor:
+  """Contiguous, with a lazy conjugation or negation carried out: the kernels read
+  the memory itself, and the cotangent of ``x.conj()`` arrives as such a view."""
+  return t.resolve_conj().resolve_neg().contiguous()
+
+
 def _stream():
   return ct.c_void_p(torch.cuda.current_stream().cuda_stream)
 
@@ -333,7 +339,7 @@ class PlaneWavePlan:
     convention for complex tensors: dL/dRe + i dL/dIm)."""
     self._check_param(w_re, "w_re")
     self._check_param(w_im, "w_im")
-    g = grad_coeff.to(self.cdtype).contiguous()
+    g = _plain(grad_coeff.to(self.cdtype))
     self._check_param(g, "grad_coeff", self.cdtype)
     gr, gi = torch.empty_like(w_re), torch.empty_like(w_im)
     st = self.lib.jrg_coeff_adjoint(self._h, _ptr(w_re), _ptr(w_im), _ptr(g), _ptr(gr), _ptr(gi),
@@ -343,6 +349,7 @@ class PlaneWavePlan:
 
   def density(self, coeff_sphere: torch.Tensor, occupation) -> torch.Tensor:
     self._check_param(coeff_sphere, "coeff", self.cdtype)
+    coeff_sphere = _plain(coeff_sphere)
     occ = self._occ(occupation)
     out = torch.empty((self.num_spin,) + self.grid, dtype=self.rdtype, device=self.device)
     st = self.lib.jrg_density(self._h, _ptr(coeff_sphere), _ptr(occ), _ptr(out),
@@ -391,7 +398,7 @@ def fft3d(x: torch.Tensor, inverse: bool = False, scale: Optional[float] = None)
     raise RuntimeError("fft3d needs a CUDA tensor (no CPU fallback)")
   if not torch.is_complex(x):
     x = x.to(torch.complex128 if x.dtype == torch.float64 else torch.complex64)
-  x = x.contiguous()
+  x = _plain(x)
   prec = 64 if x.dtype == torch.complex128 else 32
   grid = (ct.c_int * 3)(*x.shape[-3:])
   batch = int(np.prod(x.shape[:-3])) if x.dim() > 3 else 1
