@@ -94,9 +94,9 @@ __device__ __forceinline__ dc submul(dc c, dc a, dc b) {
 }
 
 // 1 / x for x > 0: approximate reciprocal, one Newton step in FP32 and one in
-// double-float
+// double-float.  The approximate division returns 0 above 2^126.
 __device__ __forceinline__ df recip(df x) {
-  float r0 = __fdividef(1.0f, x.hi);
+  float r0 = x.hi > 0x1p126f ? 1.0f / x.hi : __fdividef(1.0f, x.hi);
   r0 = fmaf(r0, fmaf(-x.hi, r0, 1.0f), r0);
   // e = 1 - x r0, r = r0 + r0 e
   const df xr = mul(x, df{r0, 0.f});
