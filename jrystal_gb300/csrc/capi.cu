@@ -14,13 +14,13 @@ namespace jrg {
 
 // ---- launchers implemented in the kernel files ----
 template <typename R> int launch_plane_inv_sphere(const jrg_plan*, const void*, void*, int, const double*, cudaStream_t);
-template <typename R> int launch_line_density(const jrg_plan*, const void*, void*, const double*, double, int, int, int, double*, cudaStream_t);
+template <typename R> int launch_line_density(const jrg_plan*, const void*, void*, const double*, double, int, int, int, double*, cudaStream_t, const int* = nullptr, int = 0);
 template <typename R> int launch_line_apply_v(const jrg_plan*, const void*, void*, const void*, int, int, const double*, cudaStream_t);
 template <typename R> int launch_plane_fwd_sphere(const jrg_plan*, const void*, const void*, void*, const double*, int, int, double, cudaStream_t);
 template <typename R> int launch_fft3d_dense(const FftAxis*, const C_t<R>*, int, int, bool, const void*, C_t<R>*, C_t<R>*, double, cudaStream_t);
 template <typename R> int launch_hartree(const jrg_plan*, const void*, C_t<R>*, C_t<R>*, double*, int, double, double, const ChargeFix&, cudaStream_t);
 template <typename R> int launch_adam_pair(const AdamArgs&, size_t, const void*, const void*, long long, cudaStream_t);
-template <typename R> int launch_pack_params(const void*, const void*, void*, int, int, int, bool, cudaStream_t);
+template <typename R> int launch_pack_params(const void*, const void*, void*, int, int, int, bool, cudaStream_t, const double* = nullptr, int* = nullptr);
 template <typename R> int launch_unpack(const void*, void*, void*, void*, int, int, int, double, cudaStream_t);
 template <typename R> int launch_gram(int, const void*, const void*, int, const void*, const void*, double2*, double2*, int, int, int, int, cudaStream_t, int* = nullptr, bool = false, int* = nullptr);
 int launch_cholesky_inv(const double2*, double2*, double2*, int, int, int*, double*, cudaStream_t, double, bool, int = 0);
@@ -779,10 +779,11 @@ static int sum_energy_slots(const jrg_plan* P, double* slots, double* energies, 
 // density of the band-major coefficients held in workspace slot c (qpart:
 // the charge partials of ChargeFix, or null).  need: weights of the bands whose
 // planes a later adjoint pass reads (a superset of the occupied ones); the
-// column kernels leave out bands of weight zero.
+// column kernels leave out bands of weight zero.  bad: nbad flags per (s,k) block
+// (density_entry), or null.
 template <typename R>
 static int density_from_c(const jrg_plan* P, const double* occ, const double* need, void* ws, void* rho_out,
-                          cudaStream_t st, double* qpart = nullptr) {
+                          cudaStream_t st, double* qpart = nullptr, const int* bad = nullptr, int nbad = 0) {
   using C = C_t<R>;
   const Workspace& w = P->ws;
   const int nsk = P->ns * P->nk;
@@ -800,7 +801,8 @@ static int density_from_c(const jrg_plan* P, const double* occ, const double* ne
       PHASE(PH_LINE_DENSITY);
       if ((rc = launch_line_density<R>(P, wsp(ws, w.t), (R*)wsp(ws, w.rho_part) + (size_t)k0 * P->ngrid, occ,
                                        1.0 / P->vol, k0 * P->nb, n * P->nb, P->nb,
-                                       (double*)wsp(ws, w.rho_scale) + k0, st)))
+                                       (double*)wsp(ws, w.rho_scale) + k0, st,
+                                       bad ? bad + (size_t)k0 * nbad : nullptr, nbad)))
         return rc;
     }
   }
@@ -1232,9 +1234,15 @@ template <typename R>
 static int density_entry(const jrg_plan* P, const void* coeff, const double* occ, void* rho, void* ws,
                          cudaStream_t st) {
   const int nsk = P->ns * P->nk;
-  int rc = launch_pack_params<R>(coeff, nullptr, wsp(ws, P->ws.c), nsk, P->ng, P->nb, true, st);
+  // The column kernels leave out bands of weight zero, whose coefficients may hold a
+  // NaN that the other kernels carry into the density: the pack leaves a flag per
+  // tile (in the Gram partials, at least 2 kB per 256 G vectors of a block and free
+  // here), and a flagged block's density scale becomes NaN.
+  int* bad = cols::active(P) ? (int*)wsp(ws, P->ws.gram_part) : nullptr;
+  const int nbad = bad ? (P->ng + 31) / 32 * ((P->nb + 31) / 32) : 0;
+  int rc = launch_pack_params<R>(coeff, nullptr, wsp(ws, P->ws.c), nsk, P->ng, P->nb, true, st, occ, bad);
   if (rc) return rc;
-  return density_from_c<R>(P, occ, occ, ws, rho, st);
+  return density_from_c<R>(P, occ, occ, ws, rho, st, nullptr, bad, nbad);
 }
 
 template <typename R>

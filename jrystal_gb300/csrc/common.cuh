@@ -62,11 +62,12 @@ __host__ __device__ inline float2 balanced_twiddle(double c, double s) {
 // w_ref with w_ref the largest |w| of w[b_begin, b_end) (ratios 0 when all are
 // zero), and, in x-block 0, gscale[grp] = w_ref * wscale.  Partials are
 // accumulated with the ratios and scaled by gscale in FP64 when reduced.
+// bad: nbad flags of the group; one that is set makes gscale NaN.
 // The caller synchronises the block before reading sw.
 template <typename R>
 __device__ __forceinline__ void group_weights(const double* __restrict__ w, int b_begin, int b_end,
                                               double wscale, double* __restrict__ gscale, int grp,
-                                              R* sw) {
+                                              R* sw, const int* __restrict__ bad = nullptr, int nbad = 0) {
   if (threadIdx.x >= 32) return;
   const int lane = threadIdx.x;
   double wref = 0.0;
@@ -74,7 +75,15 @@ __device__ __forceinline__ void group_weights(const double* __restrict__ w, int 
   for (int o = 16; o > 0; o >>= 1) wref = fmax(wref, __shfl_xor_sync(0xffffffffu, wref, o));
   const double winv = wref > 0.0 ? 1.0 / wref : 0.0;
   for (int b = b_begin + lane; b < b_end; b += 32) sw[b - b_begin] = (R)(w[b] * winv);
-  if (lane == 0 && blockIdx.x == 0) gscale[grp] = wref * wscale;
+  if (blockIdx.x == 0) {
+    int any = 0;
+    for (int i = lane; i < nbad; i += 256) {   // eight loads in flight
+#pragma unroll
+      for (int u = 0; u < 8; ++u) any |= i + 32 * u < nbad ? bad[i + 32 * u] : 0;
+    }
+    any = __any_sync(0xffffffffu, any);
+    if (lane == 0) gscale[grp] = any ? __longlong_as_double(0x7ff8000000000000LL) : wref * wscale;
+  }
 }
 
 // bytes of the group-weight array of the density kernels (16-byte aligned start)

@@ -22,7 +22,8 @@
 // Every active index of the sphere lies in the alias-free window |i| < N/4 of its
 // axis; spheres that reach further keep the plane-first kernels (k_fft_fast.cu,
 // k_fft.cu).  Bands of weight zero are left out: they add nothing to the density
-// and have no gradient.
+// and have no gradient (a caller's non-finite coefficients in such a band still
+// reach the density, see density_entry in capi.cu).
 #pragma once
 #include <algorithm>
 #include <type_traits>

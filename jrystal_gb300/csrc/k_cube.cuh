@@ -27,7 +27,7 @@ template <typename R, int N>
 __global__ void __launch_bounds__(cube_density_threads<R, N>())
 k_cube_density(C_t<R>* __restrict__ T, R* __restrict__ rho_part, const double* __restrict__ wband, double wscale,
                int band0, int nband, int bands_per_group, const short* __restrict__ col_of, int tp, int tile, int sub,
-               double* __restrict__ gscale) {
+               double* __restrict__ gscale, const int* __restrict__ bad, int nbad) {
   using C = C_t<R>;
   constexpr int H = win_half<N>(), W = win_n<N>(), parts = halves<R, N>() ? 2 : 1, M = N / parts, PV = N | 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -40,7 +40,7 @@ k_cube_density(C_t<R>* __restrict__ T, R* __restrict__ rho_part, const double* _
   const int x = blockIdx.x, grp = blockIdx.y, tid = threadIdx.x;
   const int b_begin = grp * bands_per_group, b_end = min(nband, b_begin + bands_per_group);
   live_bands(wband + band0, b_begin, b_end, list, &count);
-  group_weights<R>(wband + band0, b_begin, b_end, wscale, gscale, grp, sw);
+  group_weights<R>(wband + band0, b_begin, b_end, wscale, gscale, grp, sw, bad + (size_t)grp * nbad, nbad);
   for (int i = tid; i < W * W; i += blockDim.x) scol[i] = col_of[i];
   __syncthreads();
   const int nl = count;
@@ -153,7 +153,7 @@ template <typename R, int N> int run_cube(const jrg_plan* P, int op, const fast:
     if ((rc = prep((const void*)k_cube_density<R, N>, s.smem)) <= 0) return rc;
     k_cube_density<R, N><<<dim3(N, groups), s.threads, s.smem, st>>>(
         reinterpret_cast<C*>(const_cast<void*>(a.in)), reinterpret_cast<R*>(a.out), a.w, a.wscale, a.band0, a.nbands,
-        bpg, P->d.col_of, P->tpitch, s.tile, s.sub, a.gscale);
+        bpg, P->d.col_of, P->tpitch, s.tile, s.sub, a.gscale, a.bad, a.nbad);
     return launched("k_cube_density");
   }
   const SlabShape s = slab_shape((cube_pairs<R, N>() ? 2 : 1) * N, ylines, std::min(a.nbands, bpg), cube_apply_threads<R, N>(), [&](int tile) {

@@ -370,10 +370,10 @@ int launch_plane_inv_sphere(const jrg_plan* P, const void* coef, void* planes, i
 template <typename R>
 int launch_line_density(const jrg_plan* P, const void* planes, void* rho_part, const double* wband,
                         double wscale, int band0, int nbands, int bands_per_group, double* gscale,
-                        cudaStream_t st) {
+                        cudaStream_t st, const int* bad, int nbad) {
   using C = C_t<R>;
   {
-    fast::Args a{planes, rho_part, nullptr, wband, wscale, band0, nbands, bands_per_group, gscale};
+    fast::Args a{planes, rho_part, nullptr, wband, wscale, band0, nbands, bands_per_group, gscale, bad, nbad};
     const int f = cols::active(P) ? cols::dispatch<R>(P, fast::OP_LINE_DENSITY, a, st) : fast::dispatch<R>(P, fast::OP_LINE_DENSITY, a, st);
     if (f < 0) return -f;
     if (f > 0) return JRG_OK;
@@ -518,7 +518,7 @@ int launch_hartree(const jrg_plan* P, const void* rho, C_t<R>* mid, C_t<R>* rhog
   template int launch_plane_inv_sphere<R>(const jrg_plan*, const void*, void*, int, const double*,  \
                                           cudaStream_t);                                         \
   template int launch_line_density<R>(const jrg_plan*, const void*, void*, const double*, double, \
-                                      int, int, int, double*, cudaStream_t);                     \
+                                      int, int, int, double*, cudaStream_t, const int*, int);    \
   template int launch_line_apply_v<R>(const jrg_plan*, const void*, void*, const void*, int, int,   \
                                       const double*, cudaStream_t);                              \
   template int launch_plane_fwd_sphere<R>(const jrg_plan*, const void*, const void*, void*,        \

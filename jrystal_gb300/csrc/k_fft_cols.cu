@@ -9,7 +9,7 @@ template <typename R>
 __global__ void __launch_bounds__(kDensityThreads)
 k_slab_density(C_t<R>* __restrict__ T, R* __restrict__ rho_part, const double* __restrict__ wband, double wscale,
                int band0, int nband, int bands_per_group, const short* __restrict__ col_of, int ny, int nz, int tp,
-               int tile, int sub, double* __restrict__ gscale) {
+               int tile, int sub, double* __restrict__ gscale, const int* __restrict__ bad, int nbad) {
   using C = C_t<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const SlabLayout<R> lay(tile, ny, nz, 0, bands_per_group, true, false);
@@ -21,7 +21,7 @@ k_slab_density(C_t<R>* __restrict__ T, R* __restrict__ rho_part, const double* _
   const int x = blockIdx.x, nx = gridDim.x, grp = blockIdx.y, tid = threadIdx.x;
   const int b_begin = grp * bands_per_group, b_end = min(nband, b_begin + bands_per_group);
   live_bands(wband + band0, b_begin, b_end, list, &count);
-  group_weights<R>(wband + band0, b_begin, b_end, wscale, gscale, grp, sw);
+  group_weights<R>(wband + band0, b_begin, b_end, wscale, gscale, grp, sw, bad + (size_t)grp * nbad, nbad);
   for (int i = tid; i < window(ny) * window(nz); i += blockDim.x) scol[i] = col_of[i];
   for (int i = tid; i < ny * lay.pv; i += blockDim.x) sum[i] = (R)0;
   __syncthreads();
@@ -69,7 +69,7 @@ template <typename R> int launch_density(const jrg_plan* P, const fast::Args& a,
   const int groups = (a.nbands + a.bands_per_group - 1) / a.bands_per_group;
   k_slab_density<R><<<dim3(P->nx, groups), s.threads, s.smem, st>>>(
       reinterpret_cast<C*>(const_cast<void*>(a.in)), reinterpret_cast<R*>(a.out), a.w, a.wscale, a.band0, a.nbands,
-      a.bands_per_group, P->d.col_of, P->ny, P->nz, P->tpitch, s.tile, s.sub, a.gscale);
+      a.bands_per_group, P->d.col_of, P->ny, P->nz, P->tpitch, s.tile, s.sub, a.gscale, a.bad, a.nbad);
   return launched("k_slab_density");
 }
 
