@@ -98,8 +98,16 @@ template <int DIR, int K, int N, typename C> __device__ __forceinline__ C twmul(
         r.y = fmaf(h, ty, l * ty);
       } else {
         constexpr Pair32 w = balanced32(c, s);
-        r.x = fmaf(w.c, a.x, -w.s * a.y);
-        r.y = fmaf(w.c, a.y, w.s * a.x);
+        if constexpr (9 * k == 2 * N || 9 * k == 7 * N) {
+          // exp(+-2 pi i 2/9): the best pair is 4.6e-8 short of norm one (other ninths
+          // 2.5e-8 at most), the sine as hi + lo makes it good
+          constexpr float l = (float)(s - (double)w.s);
+          r.x = fmaf(w.c, a.x, fmaf(-w.s, a.y, -l * a.y));
+          r.y = fmaf(w.c, a.y, fmaf(w.s, a.x, l * a.x));
+        } else {
+          r.x = fmaf(w.c, a.x, -w.s * a.y);
+          r.y = fmaf(w.c, a.y, w.s * a.x);
+        }
       }
     }
     return r;
@@ -199,6 +207,12 @@ template <int N, int DIR, unsigned M, typename C> __device__ __forceinline__ voi
     sfor<H>([&](auto kk) {
       constexpr int k = kk.value + 1;
       C a = v0, b = czero<C>();
+      // sin(2 pi/5) in FP32 as hi + lo: rounded to float it is 0.4 ulp off (the other
+      // constants 0.28 at most), which scaled the density's norm by 9e-8 at 25^3 and
+      // 60^3 and by 1.1e-7 at 50^3.  The lo product comes first: added to the finished
+      // sum it would be rounded away.
+      constexpr bool lo = sizeof(R) == 4 && N == 5;
+      if constexpr (lo) b = cscale(d[k - 1], (R)(sin2pi(k * k, N) - (double)(float)sin2pi(k * k, N)));
       sfor<H>([&](auto jj) {
         constexpr int j = jj.value + 1;
         constexpr bool zp = !((M >> j) & 1) && !((M >> (N - j)) & 1);
@@ -206,7 +220,7 @@ template <int N, int DIR, unsigned M, typename C> __device__ __forceinline__ voi
           constexpr R c = (R)cos2pi(j * k, N), s = (R)sin2pi(j * k, N);
           a.x = fma(c, t[j - 1].x, a.x);
           a.y = fma(c, t[j - 1].y, a.y);
-          if constexpr (j == 1) b = cscale(d[0], s);
+          if constexpr (j == 1 && !lo) b = cscale(d[0], s);
           else { b.x = fma(s, d[j - 1].x, b.x); b.y = fma(s, d[j - 1].y, b.y); }
         }
       });
