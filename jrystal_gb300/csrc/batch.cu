@@ -51,7 +51,7 @@ struct BatchCell {
   long long* prev_idx;      // [per_step]
   double* prev_g;           // [2][per_step]
   double* prev_p;           // [2][per_step]
-  const double* coef_tab;   // [steps][2] Adam bias corrections 1 - b^t, t = 1..steps
+  const double* coef_tab;   // [steps][2] Adam factors -lr / (1 - b1^t), 1 / (1 - b2^t), t = 1..steps
   double* coef_cur;         // [2] read by k_adam
   double* hist;             // [steps][ncells][8] or null
   float* rec_x;             // [steps-1][per_step][3] of this cell
@@ -147,7 +147,7 @@ using namespace jrg;
 
 struct jrg_batch {
   int ncells = 0, steps = 0, per_step = 0, device = 0;
-  double lr = 0, b1 = 0, b2 = 0, eps = 0;
+  double b1 = 0, b2 = 0, eps = 0;
   std::vector<const jrg_plan*> plans;
   std::vector<void*> ws, params, m, v, grad;
   std::vector<const double*> occ;
@@ -233,7 +233,7 @@ int jrg_batch_create(const jrg_batch_desc* d, jrg_batch** out) {
   b->steps = d->steps;
   b->per_step = d->per_step;
   b->device = dev;
-  b->lr = d->lr; b->b1 = d->b1; b->b2 = d->b2; b->eps = d->eps;
+  b->b1 = d->b1; b->b2 = d->b2; b->eps = d->eps;
   const int nc = b->ncells, P = b->per_step, T = b->steps;
   for (int c = 0; c < nc; ++c) {
     b->plans.push_back(d->plans[c]);

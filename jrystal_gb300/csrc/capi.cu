@@ -355,17 +355,16 @@ int jrg_plan_create(const jrg_plan_desc* d, jrg_plan** out) {
     }
   }
   // column-first transforms: the (y, z) columns of the sphere in (y, z) order,
-  // their sphere entries per x, both indexed by window position (|i| < N/4
-  // when the whole sphere lies there, else every index)
+  // their sphere entries per x, both indexed by position in the window |i| < N/4
   std::vector<int> xmap;
   std::vector<short> col_of;
   {
     auto out = [](int i, int n) { const int h = (n - 1) / 4; return i > h && i < n - h; };
-    P->colwin = true;
+    bool inside = true;   // the whole sphere lies in the window
     std::vector<int> id((size_t)nyz, -1);
     for (int e = 0; e < ng; ++e) {
       const int x = (int)(gidx[e] / nyz), y = sph_yz[e] / P->nz, z = sph_yz[e] % P->nz;
-      if (out(x, P->nx) || out(y, P->ny) || out(z, P->nz)) P->colwin = false;
+      if (out(x, P->nx) || out(y, P->ny) || out(z, P->nz)) inside = false;
       id[sph_yz[e]] = 0;
     }
     P->ncol = 0;
@@ -374,11 +373,11 @@ int jrg_plan_create(const jrg_plan_desc* d, jrg_plan** out) {
     const int per16 = 16 / csize(P->prec);
     P->tpitch = (P->ncol + per16 - 1) / per16 * per16;
     P->cols = P->ncol < 32768 && (long long)P->nx * P->tpitch <= (long long)P->nact * nyz &&
-              cols::covers(P->prec, P->nx, P->ny, P->nz, P->nb, P->colwin,
+              cols::covers(P->prec, P->nx, P->ny, P->nz, P->nb, inside,
                             P->xprune && P->yzprune && P->nx == P->ny);
     if (P->cols) {
-      auto size = [&](int n) { return P->colwin ? 2 * ((n - 1) / 4) + 1 : n; };
-      auto pos = [&](int i, int n) { return (!P->colwin || i <= (n - 1) / 4) ? i : i - (n - size(n)); };
+      auto size = [](int n) { return 2 * ((n - 1) / 4) + 1; };
+      auto pos = [&](int i, int n) { return i <= (n - 1) / 4 ? i : i - (n - size(n)); };
       const int wz = size(P->nz);
       xmap.assign((size_t)size(P->nx) * P->ncol, -1);
       col_of.assign((size_t)size(P->ny) * wz, -1);

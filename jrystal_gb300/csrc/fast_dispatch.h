@@ -31,9 +31,10 @@ namespace cols {
 // column-first kernels of k_fft_cols.cu (same return convention); used when
 // active(P), for every operation of a call
 template <typename R> int dispatch(const jrg_plan* P, int op, const fast::Args& a, cudaStream_t st);
-// whether the column-first kernels take the plan's grid (pruned: the plane-first
-// ones leave out the known zeros of all axes)
-bool covers(int prec, int nx, int ny, int nz, int nb, bool colwin, bool pruned);
+// whether the column-first kernels take the plan's grid (inside: the sphere lies in
+// the window |i| < N/4 of all axes; pruned: the plane-first kernels leave out the
+// known zeros of all axes)
+bool covers(int prec, int nx, int ny, int nz, int nb, bool inside, bool pruned);
 bool active(const jrg_plan* P);
 }  // namespace cols
 }  // namespace jrg

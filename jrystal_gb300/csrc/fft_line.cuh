@@ -25,8 +25,7 @@ using reg::sin2pi;
 // widest alias-free window of a line: |i| < N/4
 template <int N> __host__ __device__ constexpr int win_half() { return (N - 1) / 4; }
 template <int N0, int H> __host__ __device__ constexpr bool in_win(int i) { return H < 0 || i <= H || i >= N0 - H; }
-// positions of a window (all of the line for H < 0), in line order
-template <int N0, int H> __host__ __device__ constexpr int win_size() { return H < 0 ? N0 : 2 * H + 1; }
+// position in the window (all of the line for H < 0), in line order
 template <int N0, int H> __host__ __device__ constexpr int win_pos(int i) { return (H < 0 || i <= H) ? i : i - (N0 - 2 * H - 1); }
 
 // ---- constants --------------------------------------------------------------
@@ -189,7 +188,6 @@ template <int N, int DIR, unsigned M, typename C> __device__ __forceinline__ voi
     // odd primes 5 and 7: sums and differences of the conjugate pairs
     constexpr int H = (N - 1) / 2;
     const C v0 = v[0];
-    constexpr bool z0 = !(M & 1);
     C t[H], d[H];
     sfor<H>([&](auto jj) {
       constexpr int j = jj.value + 1;
@@ -228,7 +226,6 @@ template <int N, int DIR, unsigned M, typename C> __device__ __forceinline__ voi
       v[k] = vadd(a, ib);
       v[N - k] = vsub(a, ib);
     });
-    (void)z0;
   }
 }
 
@@ -306,37 +303,24 @@ __device__ __forceinline__ void line_fft(L&& load, S&& store) {
 // output or input parity, is a run-time value; only the twiddles of the odd half
 // are behind a branch).  Inverse: output 2q + par is
 //   sum_n (x[n] +- x[n + M]) w_N^(par n) W_M^(n q);
-// inside the window |i| < N/4 only one of the two summands is non-zero and no
+// inside the window |i| <= H < N/4 only one of the two summands is non-zero and no
 // addition is left.  load(integral_constant<i>): input i of the window;
 // store(integral_constant<q>, v): output 2q + par.
 template <typename C, int N, int H, class L, class S>
 __device__ __forceinline__ void half_inverse(int par, L&& load, S&& store) {
-  static_assert(N % 2 == 0, "even length");
+  static_assert(N % 2 == 0 && H >= 0 && 4 * H < N, "even length, alias-free window");
   constexpr int M = N / 2;
   C a[M];
-  if constexpr (H < 0) {
-    C d[M];
-    sfor<M>([&](auto nn) {
-      constexpr int n = nn.value;
-      const C u = load(nn), v = load(std::integral_constant<int, n + M>{});
-      a[n] = vadd(u, v);
-      d[n] = vsub(u, v);
-    });
-    if (par) {
-      sfor<M>([&](auto nn) { a[nn.value] = twmul<+1, nn.value, N>(d[nn.value]); });
-    }
-  } else {
+  sfor<M>([&](auto nn) {
+    constexpr int n = nn.value, i = n <= H ? n : n + M;
+    if constexpr (in_win<M, H>(n)) a[n] = load(std::integral_constant<int, i>{});
+    else a[n] = czero<C>();
+  });
+  if (par) {
     sfor<M>([&](auto nn) {
       constexpr int n = nn.value, i = n <= H ? n : n + M;
-      if constexpr (in_win<M, H>(n)) a[n] = load(std::integral_constant<int, i>{});
-      else a[n] = czero<C>();
+      if constexpr (in_win<M, H>(n)) a[n] = twmul<+1, i, N>(a[n]);
     });
-    if (par) {
-      sfor<M>([&](auto nn) {
-        constexpr int n = nn.value, i = n <= H ? n : n + M;
-        if constexpr (in_win<M, H>(n)) a[n] = twmul<+1, i, N>(a[n]);
-      });
-    }
   }
   line_fft<C, M, +1, H>([&](auto nn) { return a[nn.value]; }, store);
 }

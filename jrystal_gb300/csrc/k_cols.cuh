@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(kColThreads, (sizeof(R) == 4 && NX <= 64) ? 6 
   }
 }
 
-// ---- T -> g_C: x forward, kinetic term, weights --------------------------------
+// ---- T -> g_C: x forward, kinetic term, weights (odd lengths) ------------------
 //   g[b][e] = w_b (tk[k][e] c[b][e] + scale FFT(V psi_b)[e])
 // Each thread copies the coefficients and kinetic values of its column to its
 // own places in shared memory while the column's T values are in flight, so
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kColThreads) k_cols_fwd(
   }
 }
 
-// The same for even lengths, two threads a column: each transforms the even or the
+// Even lengths, two threads a column: each transforms the even or the
 // odd x of the column (fft_line.cuh, half lines), they exchange through shared
 // memory what the other needs, and the even one writes the outputs k <= H, the odd
 // one k >= NX - H.  Half the registers a thread, so that more warps wait for memory
@@ -216,13 +216,14 @@ template <typename R, int N> int run_columns(const jrg_plan* P, int op, const fa
         reinterpret_cast<const C*>(a.in), reinterpret_cast<const C*>(a.aux), reinterpret_cast<C*>(a.out), a.w,
         tk_table<R>(P), P->d.xmap, P->ncol, P->tpitch, P->nb, a.band0, P->ng, P->nk, a.wscale, a.nbands, bpt);
     return launched("k_cols_fwd_pair");
+  } else {
+    const size_t sm = (sizeof(C) + sizeof(TK_t<R>) + sizeof(int)) * (size_t)win_n<N>() * kColThreads;
+    if ((rc = prep((const void*)k_cols_fwd<R, N>, sm)) <= 0) return rc;
+    k_cols_fwd<R, N><<<grid, kColThreads, sm, st>>>(
+        reinterpret_cast<const C*>(a.in), reinterpret_cast<const C*>(a.aux), reinterpret_cast<C*>(a.out), a.w,
+        tk_table<R>(P), P->d.xmap, P->ncol, P->tpitch, P->nb, a.band0, P->ng, P->nk, a.wscale, a.nbands, bpt);
+    return launched("k_cols_fwd");
   }
-  const size_t sm = (sizeof(C) + sizeof(TK_t<R>) + sizeof(int)) * (size_t)win_n<N>() * kColThreads;
-  if ((rc = prep((const void*)k_cols_fwd<R, N>, sm)) <= 0) return rc;
-  k_cols_fwd<R, N><<<grid, kColThreads, sm, st>>>(
-      reinterpret_cast<const C*>(a.in), reinterpret_cast<const C*>(a.aux), reinterpret_cast<C*>(a.out), a.w,
-      tk_table<R>(P), P->d.xmap, P->ncol, P->tpitch, P->nb, a.band0, P->ng, P->nk, a.wscale, a.nbands, bpt);
-  return launched("k_cols_fwd");
 }
 
 }  // namespace cols

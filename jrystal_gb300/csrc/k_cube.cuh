@@ -142,28 +142,37 @@ k_cube_apply_v(C_t<R>* __restrict__ T, const R* __restrict__ vr, const double* _
   }
 }
 
+// FP64 at 32^3 and 64^3 keeps the plane-first kernels (covers, k_fft_cols.cu)
+template <typename R, int N> __host__ __device__ constexpr bool cube_used() {
+  return sizeof(R) == 4 || (N != 32 && N != 64);
+}
+
 template <typename R, int N> int run_cube(const jrg_plan* P, int op, const fast::Args& a, cudaStream_t st) {
-  using C = C_t<R>;
-  const int bpg = a.bands_per_group, groups = (a.nbands + bpg - 1) / bpg;
-  constexpr int ylines = (halves<R, N>() ? 2 : 1) * win_n<N>();
-  int rc;
-  if (op == fast::OP_LINE_DENSITY) {
-    const SlabShape s = slab_shape((halves<R, N>() ? 2 : 1) * N, ylines, std::min(a.nbands, bpg), cube_density_threads<R, N>(),
-                                   [&](int tile) { return SlabLayout<R>(tile, N, N, 0, bpg, true, false).total; });
-    if ((rc = prep((const void*)k_cube_density<R, N>, s.smem)) <= 0) return rc;
-    k_cube_density<R, N><<<dim3(N, groups), s.threads, s.smem, st>>>(
-        reinterpret_cast<C*>(const_cast<void*>(a.in)), reinterpret_cast<R*>(a.out), a.w, a.wscale, a.band0, a.nbands,
-        bpg, P->d.col_of, P->tpitch, s.tile, s.sub, a.gscale, a.bad, a.nbad);
-    return launched("k_cube_density");
+  if constexpr (!cube_used<R, N>()) {
+    return 0;
+  } else {
+    using C = C_t<R>;
+    const int bpg = a.bands_per_group, groups = (a.nbands + bpg - 1) / bpg;
+    constexpr int ylines = (halves<R, N>() ? 2 : 1) * win_n<N>();
+    int rc;
+    if (op == fast::OP_LINE_DENSITY) {
+      const SlabShape s = slab_shape((halves<R, N>() ? 2 : 1) * N, ylines, std::min(a.nbands, bpg), cube_density_threads<R, N>(),
+                                     [&](int tile) { return SlabLayout<R>(tile, N, N, 0, bpg, true, false).total; });
+      if ((rc = prep((const void*)k_cube_density<R, N>, s.smem)) <= 0) return rc;
+      k_cube_density<R, N><<<dim3(N, groups), s.threads, s.smem, st>>>(
+          reinterpret_cast<C*>(const_cast<void*>(a.in)), reinterpret_cast<R*>(a.out), a.w, a.wscale, a.band0, a.nbands,
+          bpg, P->d.col_of, P->tpitch, s.tile, s.sub, a.gscale, a.bad, a.nbad);
+      return launched("k_cube_density");
+    }
+    const SlabShape s = slab_shape((cube_pairs<R, N>() ? 2 : 1) * N, ylines, std::min(a.nbands, bpg), cube_apply_threads<R, N>(), [&](int tile) {
+      return SlabLayout<R>(tile, N, N, P->ncol, bpg, false, halves<R, N>()).total;
+    });
+    if ((rc = prep((const void*)k_cube_apply_v<R, N>, s.smem)) <= 0) return rc;
+    k_cube_apply_v<R, N><<<dim3(N, groups), s.threads, s.smem, st>>>(
+        reinterpret_cast<C*>(a.out), reinterpret_cast<const R*>(a.aux), a.w, a.nbands, bpg, P->d.col_of, P->ncol,
+        P->tpitch, s.tile, s.sub);
+    return launched("k_cube_apply_v");
   }
-  const SlabShape s = slab_shape((cube_pairs<R, N>() ? 2 : 1) * N, ylines, std::min(a.nbands, bpg), cube_apply_threads<R, N>(), [&](int tile) {
-    return SlabLayout<R>(tile, N, N, P->ncol, bpg, false, halves<R, N>()).total;
-  });
-  if ((rc = prep((const void*)k_cube_apply_v<R, N>, s.smem)) <= 0) return rc;
-  k_cube_apply_v<R, N><<<dim3(N, groups), s.threads, s.smem, st>>>(
-      reinterpret_cast<C*>(a.out), reinterpret_cast<const R*>(a.aux), a.w, a.nbands, bpg, P->d.col_of, P->ncol,
-      P->tpitch, s.tile, s.sub);
-  return launched("k_cube_apply_v");
 }
 
 }  // namespace cols

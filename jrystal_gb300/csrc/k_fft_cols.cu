@@ -164,13 +164,13 @@ static bool length_ok(int n) {
   }
 }
 
-bool covers(int prec, int nx, int ny, int nz, int nb, bool colwin, bool pruned) {
+bool covers(int prec, int nx, int ny, int nz, int nb, bool inside, bool pruned) {
   // FP64 is bound by its arithmetic, and here the adjoint pass repeats the y
   // inverse: the plane-first kernels keep the cubic sizes whose known zeros they
   // leave out (32^3, 243 bands of an Al cell: 974 us for the four passes, 1085 us
   // column-first; 48^3, not pruned there: 1237 and 762 us)
   if (prec == 64 && pruned) return false;
-  if (!colwin || !length_ok(nx) || !length_ok(ny) || !length_ok(nz)) return false;
+  if (!inside || !length_ok(nx) || !length_ok(ny) || !length_ok(nz)) return false;
   // one band of either slab kernel has to fit the shared memory
   if (nb > 65535) return false;
   const int ncol = window(ny) * window(nz);

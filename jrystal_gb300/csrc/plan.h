@@ -132,10 +132,9 @@ struct jrg_plan {
   bool xprune = false;
   bool yzprune = false;
   // column-first transforms (k_fft_cols.cu): T[band][x][tpitch] over the ncol
-  // (y, z) columns that the sphere touches; colwin: every active index of all
-  // axes lies in the alias-free window |i| < N/4
+  // (y, z) columns that the sphere touches, which lies in the alias-free window
+  // |i| < N/4 of all axes
   bool cols = false;
-  bool colwin = false;
   int ncol = 0, tpitch = 0;
   double cell[9], recip[9], vol;
   std::vector<double> pos, charge, kpts;
