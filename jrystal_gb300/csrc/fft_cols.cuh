@@ -227,12 +227,13 @@ SlabShape slab_shape(int zlines, int ylines, int bands, int regs_threads, Bytes&
   return best;
 }
 
-// cubic grids with their own slab kernels (k_cube.cuh)
-#define JRG_CUBE_SIZES_0(F) F(24) F(27) F(32) F(36)
-#define JRG_CUBE_SIZES_1(F) F(40) F(45) F(48)
-#define JRG_CUBE_SIZES_2(F) F(54) F(60) F(64)
-#define JRG_CUBE_SIZES_3(F) F(72) F(80) F(96)
-#define JRG_CUBE_SIZES(F) JRG_CUBE_SIZES_0(F) JRG_CUBE_SIZES_1(F) JRG_CUBE_SIZES_2(F) JRG_CUBE_SIZES_3(F)
+// Cubic grids have slab kernels of their own (k_cube.cuh) at every length, FP64 up to
+// 63 points: above, lines by halves spill with the phases inlined (energy and gradient
+// of 48 bands: 70^3 4460 us, 4417 with the phases as functions; 72^3 3766 and 3732).
+// FP64 at 32^3 and 64^3 keeps the plane-first kernels (covers, k_fft_cols.cu).
+template <typename R, int N> __host__ __device__ constexpr bool cube_used() {
+  return sizeof(R) == 4 || (N != 32 && N <= 63);
+}
 template <typename R, int N> int run_cube(const jrg_plan* P, int op, const fast::Args& a, cudaStream_t st);
 template <typename R, int N> int run_columns(const jrg_plan* P, int op, const fast::Args& a, cudaStream_t st);
 

@@ -18,8 +18,6 @@ using C = C_t<R>;
 #elif JRG_PART_KIND == 2
 #define INST(N) template __device__ void z_apply<C, N>(Tile<C>, int, int, int, int);
 #elif JRG_PART_KIND == 4
-#undef SIZES
-#define SIZES JRG_CAT(JRG_CUBE_SIZES_, JRG_PART_CLASS)
 #define INST(N) template int run_cube<R, N>(const jrg_plan*, int, const fast::Args&, cudaStream_t);
 #else
 #define INST(N) template __device__ void z_density<C, N>(Tile<C>, int, int, int, int, int);

@@ -10,9 +10,11 @@ namespace jrg {
 namespace cols {
 
 // 168 registers hold an FP32 line of 64 of the adjoint pass, or half a line of 96
-// of either pass (density at 96^3: 2.32 ms with 256 threads, 1.46 with 384)
+// of either pass (density at 96^3: 2.32 ms with 256 threads, 1.46 with 384), or an
+// FP64 line of 32 (energy and gradient of 48 bands, 256 threads and 384: 25^3 634 and
+// 611 us, 27^3 628 and 603, 30^3 708 and 681)
 template <typename R, int N> __host__ __device__ constexpr int cube_apply_threads() {
-  return sizeof(R) == 4 ? 384 : 256;
+  return sizeof(R) == 4 || N <= 32 ? 384 : 256;
 }
 // the z phase of the adjoint pass by pairs of threads (FP64, bound by its
 // arithmetic, gains nothing: 48^3 414 us, by pairs 440)
@@ -140,11 +142,6 @@ k_cube_apply_v(C_t<R>* __restrict__ T, const R* __restrict__ vr, const double* _
       __syncthreads();
     }
   }
-}
-
-// FP64 at 32^3 and 64^3 keeps the plane-first kernels (covers, k_fft_cols.cu)
-template <typename R, int N> __host__ __device__ constexpr bool cube_used() {
-  return sizeof(R) == 4 || (N != 32 && N != 64);
 }
 
 template <typename R, int N> int run_cube(const jrg_plan* P, int op, const fast::Args& a, cudaStream_t st) {

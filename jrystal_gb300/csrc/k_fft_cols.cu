@@ -193,8 +193,8 @@ template <typename R> static int launch_columns(const jrg_plan* P, int op, const
 template <typename R> int dispatch(const jrg_plan* P, int op, const fast::Args& a, cudaStream_t st) {
   if ((op == fast::OP_LINE_DENSITY || op == fast::OP_LINE_APPLY_V) && P->nx == P->ny && P->ny == P->nz) {
     switch (P->nx) {
-#define CASE(N) case N: return run_cube<R, N>(P, op, a, st);
-      JRG_CUBE_SIZES(CASE)
+#define CASE(N) case N: if (cube_used<R, N>()) return run_cube<R, N>(P, op, a, st); break;
+      JRG_COLS_SIZES(CASE)
 #undef CASE
       default: break;
     }
