@@ -279,11 +279,11 @@ def _config(wl, n, precision=None):
           "l2": "no explicit flush: each step streams >0.9 GB of columns, coefficients and parameters, >7x the 129 MB L2"}
 
 
-# DRAM bytes (read + write) per occupied band of one k_cube_apply_v<float, 64>
-# launch, from an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum) of
-# the 64^3 Si8 cell at 2x2x2 k-points (27.1 MB for the 64 occupied bands of one
-# pipeline half; the results stay in L2); a full launch is scaled by its band count
-LINE_APPLY_V_DRAM_PER_BAND = 27.1e6 / 64
+# DRAM bytes (read + write) per occupied band of one single-stream
+# k_cube_apply_v<float, 64> launch of the 64^3 Si8 cell at 3x3x3 k-points, from an ncu
+# capture: dram__bytes_read.sum 176.8 MB + dram__bytes_write.sum 117.4 MB for 432 occupied
+# bands.  The launch writes 177 MB; the rest of it is still in L2 when it ends.
+LINE_APPLY_V_DRAM_PER_BAND = (176.8e6 + 117.4e6) / 432
 
 
 # algorithmic bytes per call of each phase of jrg_energy_grad (fused: the
@@ -543,10 +543,12 @@ def run_ours(args, wl):
                   "compulsory_bytes": int(compulsory),
                   "compulsory_frac": compulsory / (ms * 1e-3) / 1e9 / peak,
                   "fft_tflops": fft_flops / (ms * 1e-3) / 1e12}
-    roof = {"bound": "hbm", "kernel": top, "achieved": achieved, "peak": peak, "unit": "GB/s",
+    # the slab passes are bound by the arithmetic of their line transforms
+    slab = top in ("line_density", "line_apply_v")
+    roof = {"bound": f"fp{plan.precision} pipe" if slab else "hbm", "kernel": top, "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "peak_source": peak_kind, "traffic": traffic,
             "traffic_source": None if traffic is None else
-            "ncu dram bytes per band (2x2x2 k-point capture) x bands of this launch",
+            "ncu dram read + write bytes per occupied band (3x3x3 k-point capture) x bands of this launch",
             "algorithmic_bytes": pb[top], "ms_per_launch": phases[top],
             "phase_ms": {k: round(v, 4) for k, v in phases.items()}, "step_model": step_model}
     out = {"metric": METRIC, "value": 1000.0 / ms * ws, "unit": UNIT, "n_gpus": ws,
