@@ -5,7 +5,9 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
+#include <unordered_map>
 #include <vector>
 #include "fast_dispatch.h"
 #include "plan.h"
@@ -76,6 +78,33 @@ int fail(int code, const std::string& m) { g_err = m; return code; }
 int cuda_fail(cudaError_t e, const char* what) {
   g_err = std::string(what) + ": " + cudaGetErrorString(e);
   return JRG_ERR_CUDA;
+}
+
+cudaError_t allow_smem(const void* kernel, size_t bytes) {
+  struct Sizes { int fixed, most; };   // static arrays; all that a CTA can have
+  static std::mutex mu;
+  static std::unordered_map<const void*, Sizes> known;   // constants of each kernel
+  Sizes k{-1, 0};
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = known.find(kernel);
+    if (it != known.end()) k = it->second;
+  }
+  if (k.fixed < 0) {
+    int dev = 0;
+    cudaFuncAttributes a;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&k.most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+    if (e != cudaSuccess) return e;
+    k.fixed = (int)a.sharedSizeBytes;
+    std::lock_guard<std::mutex> lock(mu);
+    known[kernel] = k;
+  }
+  const long long need = (long long)bytes + k.fixed;
+  if (need > k.most) return cudaErrorInvalidValue;
+  if (need <= 48 * 1024) return cudaSuccess;   // every kernel's limit to begin with, never lowered
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, k.most - k.fixed);
 }
 
 bool factor_axis(int n, FftAxis* ax) {

@@ -184,7 +184,7 @@ inline int launched(const char* what) {
   return e == cudaSuccess ? 1 : -cuda_fail(e, what);
 }
 inline int prep(const void* kernel, size_t bytes) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  cudaError_t e = allow_smem(kernel, bytes);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)cudaSharedmemCarveoutMaxShared);

@@ -241,7 +241,7 @@ int launch_cholesky_inv_df(const double2* S, double2* Ri, int nsk, int nb, int* 
   if (sm > (size_t)optin) return 0;
   // one warp per row of the update: 8 warps up to 64 bands, 32 above
   auto go = [&](auto kern, int nt) -> cudaError_t {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem((const void*)kern, sm);
     if (e != cudaSuccess) return e;
     kern<<<nsk, nt, sm, st>>>(S, Ri, nb, flags, min_pivot, nsplit);
     return cudaSuccess;

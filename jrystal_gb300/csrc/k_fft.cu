@@ -338,7 +338,7 @@ template <typename R> size_t plane_smem(int ny, int nz, int max_rows) {
 
 template <typename K> static int set_smem(K kernel, size_t bytes) {
   if (bytes > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaError_t e = allow_smem((const void*)kernel, bytes);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(smem)");
   }
   return JRG_OK;

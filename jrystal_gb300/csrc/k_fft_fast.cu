@@ -656,7 +656,7 @@ static int optin_smem() {
 // 1: ready to launch, 0: does not fit (use the generic kernels), <0: -status
 template <typename K> static int prep(K kernel, size_t bytes) {
   if ((long long)bytes > optin_smem()) return 0;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  cudaError_t e = allow_smem((const void*)kernel, bytes);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)cudaSharedmemCarveoutMaxShared);

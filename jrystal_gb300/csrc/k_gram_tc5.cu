@@ -405,7 +405,7 @@ int launch_gram_tc5(int lay, const void* X0, const void* X1, const void* Y0, con
   const int split_len = (ng + nsplit - 1) / nsplit;
   const size_t sm = layout_for(nb).total;
   auto go = [&](auto kern) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem((const void*)kern, sm);
     if (e != cudaSuccess) return -cuda_fail(e, "cudaFuncSetAttribute(gram_tc5)");
     kern<<<dim3(nsplit, 1, nsk), kThreads, sm, st>>>(X0, X1, Y0, Y1, part, ng, nb, split_len, err);
     count_launch();

@@ -1104,7 +1104,7 @@ int launch_gram(int lx, const void* X0, const void* X1, int ly, const void* Y0, 
     auto go = [&](auto kern, int nbp) -> int {
       const size_t sm = gram_w_smem<R>(nbp, same);
       if (sm > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = allow_smem((const void*)kern, sm);
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(gram_w)");
       }
       kern<<<dim3(nsplit, 1, nsk), 256, sm, st>>>(X0, X1, Y0, Y1, part, ng, nb, split_len);
@@ -1207,7 +1207,7 @@ static int rotate_j(int lx0, const void* X0a, const void* X0b, const double2* M0
   dim3 grid((ng + 255) / 256, (nb + J - 1) / J, nsk);
   auto go = [&](auto kern) -> int {
     if (sm > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      cudaError_t e = allow_smem((const void*)kern, sm);
       if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(rotate)");
     }
     kern<<<grid, 256, sm, st>>>(X0a, X0b, M0, X1a, X1b, M1, out0, out1, ng, nb, (R)fac);
@@ -1250,7 +1250,7 @@ int launch_rotate(int out_kind, int lx0, const void* X0a, const void* X0b, const
     auto go = [&](auto kern, int nbp) -> int {
       const size_t sm = rotate_rb_smem<R>(K, nbp);
       if (sm > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = allow_smem((const void*)kern, sm);
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(rotate_rb)");
       }
       kern<<<dim3((ng + kRbGT - 1) / kRbGT, nsk), 256, sm, st>>>(X0a, X0b, M0, X1, M1, out0, out1, ng,
@@ -1297,7 +1297,7 @@ int launch_rotate_kinetic(const void* Wre, const void* Wim, const double2* Ri, v
   auto go = [&](auto kern, int nbp) -> int {
     const size_t sm = rotate_rb_smem<R>(nb, nbp);
     if (sm > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      cudaError_t e = allow_smem((const void*)kern, sm);
       if (e != cudaSuccess) return -cuda_fail(e, "cudaFuncSetAttribute(rotate_rb kinetic)");
     }
     const int nblk = (ng + kRbGT - 1) / kRbGT;
@@ -1324,7 +1324,7 @@ int launch_rotate_adam(const void* X0, const double2* M0, const void* X1, const 
   auto go = [&](auto kern, int nbp) -> int {
     const size_t sm = rotate_rb_smem<R>(2 * nb, nbp, true);
     if (sm > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      cudaError_t e = allow_smem((const void*)kern, sm);
       if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(rotate_rb adam)");
     }
     kern<<<dim3((ng + kRbGT - 1) / kRbGT, nsk), 256, sm, st>>>(X0, nullptr, M0, X1, M1, nullptr,
@@ -1485,7 +1485,7 @@ template <typename R>
 int launch_reorthonormalise(void* wr, void* wi, double2* scratch, int nsk, int ng, int nb, cudaStream_t st) {
   const size_t sm = (size_t)nb * sizeof(double);
   if (sm > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_reorthonormalise<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem((const void*)k_reorthonormalise<R>, sm);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_reorthonormalise)");
   }
   k_reorthonormalise<R><<<nsk, kReorthThreads, sm, st>>>(reinterpret_cast<R*>(wr), reinterpret_cast<R*>(wi),

@@ -362,7 +362,7 @@ int launch_rotate_tc(int out_kind, int lx0, const void* X0a, const void* X0b, co
   const size_t sm = sizeof(float) * ((size_t)128 * (KP + 4) + 2 * (size_t)KP * (NP + 8));
   dim3 grid((ng + 127) / 128, nsk);
   auto go = [&](auto kern) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem((const void*)kern, sm);
     if (e != cudaSuccess) return -cuda_fail(e, "cudaFuncSetAttribute(k_rotate_tc)");
     kern<<<grid, 256, sm, st>>>(X0a, X0b, X1, bscratch, out0, out1, ng, nb, KP, NP, (float)fac);
     count_launch();

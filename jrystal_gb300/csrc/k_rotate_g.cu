@@ -364,7 +364,7 @@ static int rg_go(const void* X0a, const void* X0b, const double2* M0, const void
   const bool vout = (OUT == RG_GMAJOR_SPLIT || OUT == RG_ADAM) && nb % 4 == 0 && NJ % 4 == 0 && sizeof(R) == 4;
   auto go = [&](auto kern) -> int {
     if (sm > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      cudaError_t e = allow_smem((const void*)kern, sm);
       if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_rotate_g)");
     }
     const dim3 grid((nb + NJ - 1) / NJ, (ng + kRgThreads * TG - 1) / (kRgThreads * TG), nsk);

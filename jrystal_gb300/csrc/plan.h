@@ -20,6 +20,13 @@ int cuda_fail(cudaError_t e, const char* what);
 
 void count_launch();
 
+// Lets the kernel have all the dynamic shared memory of a CTA beside its static
+// arrays (bytes: what the launch takes; more than there is: cudaErrorInvalidValue).
+// The limit is the kernel's, not the launch's: set to each launch's own need, a
+// smaller plan on another thread lowers it between this thread's call and its launch,
+// which is then refused.
+cudaError_t allow_smem(const void* kernel, size_t bytes);
+
 #define JRG_LAUNCH_CHECK(what)                           \
   do {                                                   \
     ::jrg::count_launch();                               \
