@@ -146,7 +146,8 @@ int jrg_coeff_adjoint(const jrg_plan* plan, const void* w_re, const void* w_im,
 
 /* Occupation-weighted density on the grid from sphere coefficients.
  * coeff: [S][K][G][B] complex; occupation: device double [S][K][B];
- * density: [S][nx][ny][nz] real. */
+ * density: [S][nx][ny][nz] real.  A non-finite coefficient makes the density of
+ * its spin NaN, also in a band of occupation zero. */
 int jrg_density(const jrg_plan* plan, const void* coeff, const double* occupation,
                 void* density, void* workspace, cudaStream_t stream);
 

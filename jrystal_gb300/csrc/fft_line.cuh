@@ -4,7 +4,8 @@
 // memory, no barrier, no twiddle table.  The transform is a mixed-radix
 // decimation in time, N = P*Q recursively down to radices 2, 3, 4, 5, 7 and
 // 8, fully unrolled; twiddles are compile-time constants (FP32: the
-// norm-balanced pair of common.cuh's balanced_twiddle).
+// norm-balanced pair of common.cuh's balanced_twiddle, and hi + lo where no pair of
+// floats comes near norm one).
 //
 // WIN: the half width H of the window of non-zero inputs (|i| <= H, counted
 // cyclically; H < 0: every input).  The additions of the known zeros are left
